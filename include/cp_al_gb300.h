@@ -109,7 +109,8 @@ typedef struct {
                                      TMA bulk copies while they work on the current one: 1 = its
                                      matrix slice, 2 = also its rows' epilogue inputs, 0 = off
                                      (a block per row block, loads issued by the threads);
-                                     -1 (default) = off.  Results are bit-identical in every mode */
+                                     -1 (default) = off, and persistent_loop may replace the launches.
+                                     Results are bit-identical in modes 0, 1 and 2 */
     int infeasibility_detection;  /* nonzero: at every evaluation, test the iterates' displacement from
                                      the restart anchor as infeasibility certificates and stop with
                                      TERMINATION_REASON_PRIMAL_INFEASIBLE or _DUAL_INFEASIBLE (the ray
@@ -117,13 +118,14 @@ typedef struct {
                                      (LP/CP_AL/src/utils.cu:919-1029, 281-297) but never calls them:
                                      default 0, as there.  Single-LP solver only */
     double eps_infeasible;        /* tolerance of those tests (default 1e-8) */
-    int persistent_loop;          /* small LPs: run the iteration, evaluation and restart loop inside one
-                                     cooperative launch (grid barriers between the products) instead of a
-                                     CUDA graph of per-iteration launches.  1 = when the problem allows it
-                                     (row blocks of at most 1,024 nonzeros, no column panels, staged or
-                                     hot-row product, restart target selection, infeasibility detection or
-                                     timing); 0 or -1 (default) = never (measured no faster than the
-                                     graph path with programmatic launches, which hides the launches) */
+    int persistent_loop;          /* LPs whose matrices fit in the shared memory of the GPU's SMs: run an
+                                     evaluation block's iterations, and the FP64 power iteration, in one
+                                     resident launch each instead of one launch per product.  -1 (default)
+                                     = where that was measured faster (by size and precision; not with
+                                     column panels, an explicit primal_staged or timing); 1 = the
+                                     iterations of every LP that fits, with the launches' summation
+                                     order (bit-identical to 0), the power iteration by launches; 0 =
+                                     never */
     int dual_fused_finish;        /* with the panel path: the group that writes a long row's last panel
                                      partial also sums the row's partials (fixed order) and runs its
                                      dual epilogue, instead of a separate launch.  1 = fused; 0 or -1

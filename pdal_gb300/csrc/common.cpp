@@ -182,6 +182,106 @@ HostPlan plan_rows(int nr, const int *rp, int S) {
     return P;
 }
 
+HostSlices plan_slices(const HostPlan &P, const int *rp, int lanes) {
+    HostSlices Q;
+    /* lanes per row of a STREAM block, as rowblock_run_at chooses them */
+    auto group = [&](int nrows) {
+        if (lanes > 0) return lanes;
+        int g = 32;
+        while (g > 1 && g * nrows > kThreads) g >>= 1;
+        return g;
+    };
+    /* the blocks, STREAM blocks merged into windows where the lanes are given */
+    std::vector<std::pair<int, int>> win; /* {first row, end row}, or {block, -1} of a long piece */
+    for (int b = 0; b < P.nblocks; ++b) {
+        const int *d = &P.desc[4 * (size_t)b];
+        if (d[1] < d[0])
+            win.emplace_back(b, -1);
+        else if (lanes > 0 && !win.empty() && win.back().second == d[0] && d[1] - win.back().first <= 1024)
+            win.back().second = d[1];
+        else
+            win.emplace_back(d[0], d[1]);
+    }
+    const int nw = (int)win.size();
+    std::vector<int> first((size_t)nw + 1, 0);
+    for (int b = 0; b < nw; ++b) {
+        const int nrows = win[b].second - win[b].first;
+        first[b + 1] = first[b] + (win[b].second < 0 ? 8 : (nrows * group(nrows) + 31) / 32);
+    }
+    Q.n = first[nw];
+    Q.desc.resize(4 * (size_t)Q.n);
+    Q.rl.assign(64 * (size_t)Q.n, 0);
+    const int nt = host_threads(32LL * Q.n);
+    parallel_for(nt, [&](int t) {
+        std::vector<std::pair<int, int>> rows; /* {-length, row}: longest first, ties in row order */
+        std::vector<int> at;                   /* counting sort by length */
+        for (int b = (int)((long long)nw * t / nt); b < (int)((long long)nw * (t + 1) / nt); ++b) {
+            if (win[b].second < 0) { /* a piece of a long row: 256 virtual threads, their entries 256 apart */
+                const int *d = &P.desc[4 * (size_t)win[b].first];
+                const int lid = ~d[1], cnt = d[3] - d[2];
+                const int piece = (d[2] - P.linfo[4 * (size_t)lid + 3]) / P.S;
+                for (int w = 0; w < 8; ++w) {
+                    const size_t s = (size_t)first[b] + w;
+                    Q.desc[4 * s + 1] = (std::max(cnt - 32 * w, 0) + kThreads - 1) / kThreads;
+                    Q.desc[4 * s + 2] = 0;
+                    Q.desc[4 * s + 3] = (P.linfo[4 * (size_t)lid + 2] + piece) * 8 + w;
+                    for (int l = 0; l < 32; ++l) {
+                        Q.rl[64 * s + 2 * l] = lid;
+                        Q.rl[64 * s + 2 * l + 1] = (std::max(cnt - 32 * w - l, 0) + kThreads - 1) / kThreads;
+                    }
+                }
+                continue;
+            }
+            const int nrows = win[b].second - win[b].first, g = group(nrows), per = 32 / g;
+            int longest = 0;
+            for (int r = win[b].first; r < win[b].second; ++r) longest = std::max(longest, rp[r + 1] - rp[r]);
+            at.assign((size_t)longest + 2, 0);
+            for (int r = win[b].first; r < win[b].second; ++r) at[longest - (rp[r + 1] - rp[r]) + 1]++;
+            for (int q = 0; q <= longest; ++q) at[q + 1] += at[q];
+            rows.resize(nrows);
+            for (int r = win[b].first; r < win[b].second; ++r)
+                rows[at[longest - (rp[r + 1] - rp[r])]++] = {rp[r] - rp[r + 1], r};
+            for (int q = 0; q < nrows; q += per) {
+                const size_t s = (size_t)first[b] + q / per;
+                Q.desc[4 * s + 1] = (-rows[q].first + g - 1) / g;
+                Q.desc[4 * s + 2] = g;
+                Q.desc[4 * s + 3] = 0;
+                for (int l = 0; l < 32; ++l) {
+                    const bool in = q + l / g < nrows;
+                    Q.rl[64 * s + 2 * l] = in ? rows[q + l / g].second : -1;
+                    Q.rl[64 * s + 2 * l + 1] = in ? std::max(-rows[q + l / g].first - l % g + g - 1, 0) / g : 0;
+                }
+            }
+        }
+    });
+    for (int s = 0; s < Q.n; ++s) {
+        if (Q.len > (long long)INT32_MAX - 65536) throw Error("matrix too large for a sliced plan");
+        Q.desc[4 * (size_t)s] = (int)Q.len;
+        Q.len += 32LL * Q.desc[4 * (size_t)s + 1];
+    }
+    return Q;
+}
+
+std::vector<int> split_slices(const HostSlices &Q, int parts, long long &most) {
+    /* a slice costs its entries and about four more for its epilogue */
+    std::vector<int> cut((size_t)parts + 1, Q.n);
+    const long long total = Q.len / 32 + 4LL * Q.n;
+    long long done = 0;
+    int b = 0;
+    most = 0;
+    for (int s = 0; s < Q.n; ++s) {
+        while (b < parts && done >= total * b / parts) cut[b++] = s;
+        done += Q.desc[4 * (size_t)s + 1] + 4;
+    }
+    while (b < parts) cut[b++] = Q.n;
+    for (int p = 0; p < parts; ++p) {
+        const long long k0 = cut[p] < Q.n ? Q.desc[4 * (size_t)cut[p]] : Q.len;
+        const long long k1 = cut[p + 1] < Q.n ? Q.desc[4 * (size_t)cut[p + 1]] : Q.len;
+        most = std::max(most, k1 - k0);
+    }
+    return cut;
+}
+
 HostPanels plan_panels(int nr, int nc, const int *rp, const int *ci, int S, int W, int target_blocks) {
     HostPanels Q;
     Q.W = W;

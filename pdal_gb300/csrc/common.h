@@ -116,6 +116,22 @@ struct HostPlan {
 };
 HostPlan plan_rows(int nr, const int *rp, int S);
 
+/* The same rows as 32-lane slices (slices.cuh): a warp's worth of lane lists,
+ * stored lane-major. */
+struct HostSlices {
+    int n = 0;             /* slices */
+    long long len = 0;     /* packed entries, padding of short lanes included */
+    std::vector<int> desc; /* 4 ints per slice: {first entry, entries of the longest lane, g, slot} */
+    std::vector<int> rl;   /* 2 ints per lane: {row or long row id (-1: none), entries} */
+};
+/* `lanes` = 0: a row's lanes are those of rowblock_run_at (bit-identical
+ * sums); > 0: that many lanes (a power of two) for every row that is not
+ * long, over windows of 1,024 rows sorted by length. */
+HostSlices plan_slices(const HostPlan &P, const int *rp, int lanes);
+/* First slice of each of `parts` contiguous ranges of about equal cost
+ * (parts + 1 entries), and the largest number of packed entries in one. */
+std::vector<int> split_slices(const HostSlices &Q, int parts, long long &most);
+
 /*
  * Column-panel plan of the long rows (more than S nonzeros) of a CSR matrix,
  * for the dual product A x of a matrix whose long rows hold much of its

@@ -1495,199 +1495,6 @@ __global__ void k_restart(const CpalState *__restrict__ st, int n, int m, const 
 static __global__ void k_start_clock(CpalState *st) { st->t_start_ns = globaltimer_ns(); }
 
 /* ------------------------------------------------------------------ */
-/* small LPs: the whole loop in one cooperative launch                 */
-/* ------------------------------------------------------------------ */
-/* A small LP's iteration is a few microseconds of work spread over a few
- * hundred blocks, so two kernel launches per iteration (even inside a CUDA
- * graph) cost as much as the work.  k_cpal_loop runs evaluation blocks
- * entirely on the device: every block of the grid (all co-resident, launched
- * cooperatively) walks the row blocks of each product, and a grid barrier
- * separates the primal product, the dual product, the evaluation, the
- * controller (block 0) and the restart.  The row-block bodies, epilogues,
- * controller and restart are the graph path's, with one difference: vectors
- * written inside the launch are gathered through L2 (__ldcg), never through
- * the read-only path. */
-struct LoopBar {
-    unsigned int count, gen;
-    int err, pad;
-};
-
-__device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-/* Grid barrier number `k` (1, 2, ... within the launch; the counter is zero
- * at launch): one release-add per block on a monotonic counter, then an
- * acquire spin until all blocks of the k-th barrier have arrived.  False,
- * with the barrier marked failed for every block, when a wait exceeds
- * `limit` polls. */
-__device__ __forceinline__ bool loop_sync(LoopBar *b, unsigned k, long long limit, int *sok) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        const unsigned target = k * gridDim.x;
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&b->count) : "memory");
-        long long spins = 0;
-        while (ld_acquire_gpu(&b->count) < target) {
-            if (++spins > limit) {
-                atomicExch(&b->err, 1);
-                ok = 0;
-                break;
-            }
-            if ((spins & 1023) == 0 && *(volatile int *)&b->err) {
-                ok = 0;
-                break;
-            }
-        }
-        *sok = ok;
-    }
-    __syncthreads();
-    return *sok != 0;
-}
-
-template <typename T>
-struct LoopArgs {
-    RowPlanDev at_it, a_it, at_ev, a_ev;
-    const int *at_rp, *at_ci, *a_rp, *a_ci;
-    const T *at_val, *a_val;      /* iteration values (the form's precision) */
-    const double *at_v64, *a_v64; /* evaluation values */
-    PrimalArgs<T> pa;
-    DualArgs<T> da;
-    const T *gat; /* gathered by the primal product: u (beta > 0) or y */
-    EvalRowArgs<T> ra;
-    EvalColArgs<T> ca;
-    CpalState *st;
-    CpalParams p;
-    HalpernW *wt;
-    HalpernWf *wtf;
-    int nrow_slots, ncol_slots;
-    int n, m;
-    double *x0, *y0, *ax0;
-    float2 *x0f, *y0f, *ax0f;
-    const double *phat;
-    LoopBar *bar;
-    long long spin_limit;
-    int max_blocks; /* evaluation blocks before the launch returns to the host */
-    int *err;
-};
-
-template <typename T>
-__device__ __forceinline__ const typename WeightT<T>::type &loop_weight(const LoopArgs<T> &L, int i);
-template <>
-__device__ __forceinline__ const HalpernW &loop_weight<double>(const LoopArgs<double> &L, int i) {
-    return L.wt[i];
-}
-template <>
-__device__ __forceinline__ const HalpernWf &loop_weight<float>(const LoopArgs<float> &L, int i) {
-    return L.wtf[i];
-}
-
-template <typename T, int S, bool MAJOR>
-__device__ __forceinline__ void loop_primal(const LoopArgs<T> &L, const Coefs<T> &k, int i,
-                                            RowBlockSmem<S, 1, T> &sm) {
-    PrimalEpi<T, MAJOR> epi;
-    epi.a = L.pa;
-    epi.k = k;
-    epi.w = loop_weight<T>(L, i).w;
-    epi.omw = loop_weight<T>(L, i).omw;
-    const T *gat = L.gat;
-    auto g = [&](int c, T *out) { out[0] = __ldcg(gat + c); };
-    Red<0, 0> red;
-    for (int blk = blockIdx.x; blk < L.at_it.nblocks; blk += gridDim.x) {
-        rowblock_run_at<S, 1, T>(blk, L.at_it, L.at_rp, L.at_ci, L.at_val, g, epi, red, sm);
-        __syncthreads();
-    }
-}
-
-template <typename T, int S, bool MAJOR, bool BETA>
-__device__ __forceinline__ void loop_dual(const LoopArgs<T> &L, const Coefs<T> &k, int i,
-                                          RowBlockSmem<S, 1, T> &sm) {
-    DualEpi<T, MAJOR, BETA> epi;
-    epi.a = L.da;
-    epi.k = k;
-    epi.w = loop_weight<T>(L, i).w;
-    epi.omw = loop_weight<T>(L, i).omw;
-    const T *xbar = L.pa.xbar;
-    auto g = [&](int c, T *out) { out[0] = __ldcg(xbar + c); };
-    Red<0, 0> red;
-    for (int blk = blockIdx.x; blk < L.a_it.nblocks; blk += gridDim.x) {
-        rowblock_run_at<S, 1, T>(blk, L.a_it, L.a_rp, L.a_ci, L.a_val, g, epi, red, sm);
-        __syncthreads();
-    }
-}
-
-template <typename T, int S, int SE, bool BETA>
-__global__ void __launch_bounds__(kThreads) k_cpal_loop(LoopArgs<T> L) {
-    constexpr size_t B1 = sizeof(RowBlockSmem<S, 1, T>), B2 = sizeof(RowBlockSmem<SE, 3, double>),
-                     B3 = sizeof(RowBlockSmem<SE, 2, double>);
-    constexpr size_t BM = B1 > B2 ? (B1 > B3 ? B1 : B3) : (B2 > B3 ? B2 : B3);
-    __shared__ __align__(16) unsigned char raw[BM];
-    __shared__ double sbuf[11 * (kThreads / 32)];
-    __shared__ int sok, sflag;
-    auto &smi = *reinterpret_cast<RowBlockSmem<S, 1, T> *>(raw);
-    auto &smr = *reinterpret_cast<RowBlockSmem<SE, 3, double> *>(raw);
-    auto &smc = *reinterpret_cast<RowBlockSmem<SE, 2, double> *>(raw);
-    const int F = L.p.F;
-    auto give_up = [&]() {
-        if (threadIdx.x == 0) {
-            atomicExch(L.err, 2);
-            atomicExch(&L.st->status, kStatusDeviceError);
-        }
-    };
-    unsigned nsync = 0;
-#define PDAL_LOOP_SYNC()                                                                                               \
-    do {                                                                                                               \
-        if (!loop_sync(L.bar, ++nsync, L.spin_limit, &sok)) {                                                          \
-            give_up();                                                                                                 \
-            return;                                                                                                    \
-        }                                                                                                              \
-    } while (0)
-    for (int blocks = 0; blocks < L.max_blocks; ++blocks) {
-        /* every block reads the state after the same barrier */
-        if (threadIdx.x == 0) sflag = L.st->status;
-        __syncthreads();
-        if (sflag) return;
-        Coefs<T> k;
-        load_coefs(L.st, k);
-        for (int i = 1; i <= F; ++i) {
-            if (i == F)
-                loop_primal<T, S, true>(L, k, i, smi);
-            else
-                loop_primal<T, S, false>(L, k, i, smi);
-            PDAL_LOOP_SYNC();
-            if (i == F)
-                loop_dual<T, S, true, BETA>(L, k, i, smi);
-            else
-                loop_dual<T, S, false, BETA>(L, k, i, smi);
-            PDAL_LOOP_SYNC();
-        }
-        for (int blk = blockIdx.x; blk < L.a_ev.nblocks; blk += gridDim.x) {
-            eval_rows_at<T, SE, false>(blk, L.a_ev, L.a_rp, L.a_ci, L.a_v64, L.ra, smr);
-            __syncthreads();
-        }
-        for (int blk = blockIdx.x; blk < L.at_ev.nblocks; blk += gridDim.x) {
-            eval_cols_at<T, SE, false, false>(blk, L.at_ev, L.at_rp, L.at_ci, L.at_v64, L.ca, smc);
-            __syncthreads();
-        }
-        PDAL_LOOP_SYNC();
-        if (blockIdx.x == 0)
-            control_block(L.ra.part, L.nrow_slots, L.ca.part, L.ncol_slots, nullptr, 0, nullptr, 0, L.st, L.p, L.wt,
-                          L.wtf, sbuf);
-        PDAL_LOOP_SYNC();
-        restart_all<T, BETA>(L.st, L.n, L.m, L.pa.xh, L.pa.x, L.x0, L.x0f, L.da.yh, L.da.y, L.y0, L.y0f, L.phat,
-                             L.da.ax, L.ax0, L.ax0f, L.da.u, L.da.lb, L.da.ub, L.pa.xbar, L.da.ybar);
-        PDAL_LOOP_SYNC();
-        /* the end of the FP32 phase is the host's to carry out */
-        if (threadIdx.x == 0) sflag = L.st->phase_switch;
-        __syncthreads();
-        if (sflag) return;
-    }
-#undef PDAL_LOOP_SYNC
-}
-
-/* ------------------------------------------------------------------ */
 /* result (LP/CP_AL/src/solver.cu:1768-1793, 2481-2500)                 */
 /* ------------------------------------------------------------------ */
 struct ResultColEpi : NoLongRed {

@@ -17,6 +17,7 @@
 #include "../../include/cp_al_gb300.h"
 #include "common.h"
 #include "cpal_kernels.cuh"
+#include "slices.cuh"
 #include "cpal_setup.h"
 
 #include <algorithm>
@@ -285,13 +286,58 @@ class CpalSolver {
     std::vector<int> eq_long_h_[2];
     int *eq_long_[2] = {nullptr, nullptr}; /* [A, A^T] */
     void setup_staged();
-    /* the persistent cooperative loop (k_cpal_loop) for small LPs */
-    bool use_loop_ = false;
-    int loop_grid_[2] = {0, 0}; /* [FP64?] */
-    LoopBar *loop_bar_ = nullptr;
-    void setup_loop();
+    /* LPs that fit on the chip: sliced copies of A^T and A (index 0, 1) in each
+     * precision (FP32, FP64), the iterations of an evaluation block and the
+     * sigma_max estimate as resident launches (slices.cuh) */
+    struct Sliced {
+        HostSlices h;
+        std::vector<int> cut;
+        int4 *desc = nullptr;
+        int2 *rl = nullptr;
+        int *ci = nullptr, *cta = nullptr;
+        void *val = nullptr;
+        ulonglong2 *part = nullptr;
+    } sl_[2][2];
+    int flow_grid_ = 0;             /* CTAs of the resident launches */
+    int flow_shift_[2] = {0, 0};    /* spacing of the tagged x-bar and u */
     template <typename T>
-    void launch_loop(int max_blocks);
+    TaggedVec<T> tagged_x() const {
+        return TaggedVec<T>{(typename Tagged<T>::Word *)flow_xt_, flow_shift_[0]};
+    }
+    template <typename T>
+    TaggedVec<T> tagged_u() const {
+        return TaggedVec<T>{(typename Tagged<T>::Word *)flow_ut_, flow_shift_[1]};
+    }
+    unsigned *flow_bar_ = nullptr;
+    size_t flow_smem_[2] = {0, 0};  /* shared memory of a CTA, 0: the precision runs one launch per product */
+    ulonglong2 *flow_xt_ = nullptr, *flow_ut_ = nullptr, *flow_sums_ = nullptr; /* tagged words */
+    void plan_flow();
+    void alloc_flow();
+    void upload_flow();
+    void pack_flow();
+    void clear_flow();
+    enum class Flow { launches, tagged, barrier };
+    /* How the iteration's products run.  The lines lie where the measured
+     * times cross (the table in slices.cuh): polling pays up to about 90,000
+     * nonzeros in both precisions; above, FP64 gains from the resident form
+     * at every size that fits, FP32, whose launches take half the time, from
+     * about 600,000 on.  `timing` brackets single launches. */
+    template <typename T>
+    Flow flow_form() const {
+        if (flow_smem_[sizeof(T) == 8] == 0 || O_.timing != 0) return Flow::launches;
+        if (nnz_ <= 90000 || O_.persistent_loop == 1) return Flow::tagged;
+        return sizeof(T) == 8 || nnz_ >= 600000 ? Flow::barrier : Flow::launches;
+    }
+    template <typename T>
+    SliceDev<T> slice_dev(int which) const;
+    template <typename T>
+    FlowPowerArgs<T> power_args();
+    template <typename T>
+    void launch_flow(int F);
+    template <typename... K, typename... A>
+    void launch_coop(void (*kern)(K...), int threads, size_t smem, A... args);
+    /* polls of an L2 round trip each: a wait gives up after about 2 s */
+    FlowGuard guard() const { return FlowGuard{dev_err_, 1 << 22}; }
     bool staged_rows() const { return O_.primal_staged == 2; }
     void check_device_error();
     int *At_ci_hot_ = nullptr;
@@ -593,7 +639,7 @@ void CpalSolver::alloc_all() {
     for (int q = 0; q < 2; ++q) eq_long_[q] = arena_.take<int>(std::max<size_t>(eq_long_h_[q].size(), 1));
     if (device_transpose_) at_cursor_ = arena_.take<int>(n + 1);
     if (device_transpose_ && use_hot_) hot_id_d_ = arena_.take<int>(std::max<size_t>(m, 1));
-    loop_bar_ = arena_.take<LoopBar>(1);
+    alloc_flow();
     if (use_panels_) {
         const size_t len = (size_t)pan_host_.len, hp = (size_t)pan_host_.H * pan_host_.P;
         const size_t n1 = std::max<size_t>(sh_r1_h.size(), 1), n2 = std::max<size_t>(sh_r2_h.size(), 1),
@@ -742,67 +788,143 @@ void CpalSolver::setup_staged() {
     });
 }
 
-/* The persistent loop runs small LPs (row blocks of at most 1,024 nonzeros)
- * on the default iteration path: no column panels, staged or hot-row primal
- * product, restart target selection, infeasibility rays or per-launch
- * timing, all of which the graph path carries.  Its grid is what the device
- * holds at once (a cooperative launch), capped by the work. */
-#define PDAL_WITH_S_LOOP(Sval, ...)                   \
-    switch (Sval) {                                   \
-    case 256: {                                       \
-        constexpr int SL = 256;                       \
-        __VA_ARGS__;                                  \
-    } break;                                          \
-    case 512: {                                       \
-        constexpr int SL = 512;                       \
-        __VA_ARGS__;                                  \
-    } break;                                          \
-    case 1024: {                                      \
-        constexpr int SL = 1024;                      \
-        __VA_ARGS__;                                  \
-    } break;                                          \
-    default:                                          \
-        throw Error("persistent loop: unsupported row-block budget"); \
-    }
+/* Resident launches need the packed matrices of both products in the shared
+ * memory of one CTA per SM, in the precision that iterates. */
+constexpr size_t kFlowSmem = 224 * 1024;
 
-void CpalSolver::setup_loop() {
-    const bool eligible = S_it_ <= 1024 && S_ev_ == S_it_ && !use_panels_ && !use_hot_ && !use_staged_ &&
-                          cp_.restart_select == 0 && !cp_.infeas && O_.timing == 0 && !cp_.pulse && !cp_.trigger &&
-                          !cp_.dyn;
-    const bool want = O_.persistent_loop == 1;
-    use_loop_ = eligible && want;
-    if (!use_loop_) return;
+void CpalSolver::plan_flow() {
+    flow_grid_ = 0;
+    flow_smem_[0] = flow_smem_[1] = 0;
+    if (O_.persistent_loop == 0 || m_ == 0 || nnz_ == 0 || use_panels_ || O_.primal_staged >= 0) return;
     int dev = 0, sms = 0, coop = 0;
     PDAL_CUDA(cudaGetDevice(&dev));
     PDAL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     PDAL_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    if (!coop) {
-        use_loop_ = false;
-        return;
-    }
-    const long long work = std::max({(long long)At_.it.hp.nblocks, (long long)A_.it.hp.nblocks,
-                                     (long long)At_.ev.hp.nblocks, (long long)A_.ev.hp.nblocks,
-                                     ((long long)std::max(n_, m_) + kThreads - 1) / kThreads, 1LL});
-    auto wave = [&](auto kernel) {
-        int occ = 0;
-        PDAL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kThreads, 0));
-        if (occ < 1) throw Error("persistent loop does not fit on one SM");
-        return (int)std::min<long long>((long long)occ * sms, work);
-    };
-    PDAL_WITH_S_LOOP(S_it_, {
-        if (beta_on_) {
-            loop_grid_[0] = wave(k_cpal_loop<float, SL, SL, true>);
-            loop_grid_[1] = wave(k_cpal_loop<double, SL, SL, true>);
-        } else {
-            loop_grid_[0] = wave(k_cpal_loop<float, SL, SL, false>);
-            loop_grid_[1] = wave(k_cpal_loop<double, SL, SL, false>);
+    if (!coop) return;
+    flow_grid_ = sms;
+    /* a short vector is spread out: entries of one line written by several
+     * SMs while many poll it cost several exchanges' time (40,000 + 400 entries,
+     * exchange alone: 26,900 cycles packed, 6,600 with 128 bytes per entry) */
+    for (int q = 0; q < 2; ++q) flow_shift_[q] = (q ? m_ : n_) <= 1024 ? 4 : (q ? m_ : n_) <= 4096 ? 2 : 0;
+    for (int f = fp32_phase_ ? 0 : 1; f < 2; ++f) {
+        const size_t entry = sizeof(int) + (f ? sizeof(double) : sizeof(float));
+        if ((size_t)nnz_ * 2 * entry > sms * kFlowSmem) continue;
+        size_t bytes = 0;
+        for (int q = 0; q < 2; ++q) {
+            Sliced &l = sl_[f][q];
+            const int nr = q ? m_ : n_;
+            /* as few lanes per row as give every SM a slice */
+            int lanes = 0;
+            if (O_.persistent_loop != 1)
+                for (lanes = 1; lanes < 32 && (long long)nr * lanes < 32LL * sms && 2LL * lanes * nr <= nnz_;) lanes *= 2;
+            l.h = plan_slices((q ? A_ : At_).it.hp, q ? prob_->constraint_matrix_row_pointers : At_host_.rp.data(),
+                              lanes);
+            long long most = 0;
+            l.cut = split_slices(l.h, sms, most);
+            bytes += (size_t)most * entry;
         }
-    });
-    PDAL_CUDA(cudaMemsetAsync(loop_bar_, 0, sizeof(LoopBar), stream_));
+        if (bytes <= kFlowSmem) flow_smem_[f] = std::max<size_t>(bytes, 16);
+    }
 }
 
-/* A device wait that ran out (a staging wait of k_primal_tma, a grid
- * barrier of k_cpal_loop) stops the solve (status kStatusDeviceError) and is
+void CpalSolver::alloc_flow() {
+    for (int f = 0; f < 2; ++f)
+        for (int q = 0; q < 2 && flow_smem_[f]; ++q) {
+            Sliced &l = sl_[f][q];
+            const size_t len = (size_t)std::max(l.h.len, 1LL);
+            l.desc = arena_.take<int4>(std::max(l.h.n, 1));
+            l.rl = arena_.take<int2>(32 * (size_t)std::max(l.h.n, 1));
+            l.cta = arena_.take<int>((size_t)flow_grid_ + 1);
+            l.ci = arena_.take<int>(len);
+            l.val = f ? (void *)arena_.take<double>(len) : (void *)arena_.take<float>(len);
+            l.part = arena_.take<ulonglong2>(8 * (size_t)std::max((q ? A_ : At_).it.hp.npieces, 1));
+        }
+    if (flow_smem_[0] || flow_smem_[1]) {
+        flow_xt_ = arena_.take<ulonglong2>((size_t)n_ << flow_shift_[0]);
+        flow_ut_ = arena_.take<ulonglong2>((size_t)m_ << flow_shift_[1]);
+        flow_bar_ = arena_.take<unsigned>(1);
+        flow_sums_ = arena_.take<ulonglong2>(32 * (size_t)flow_grid_);
+    }
+}
+
+void CpalSolver::upload_flow() {
+    auto up = [&](void *dst, const std::vector<int> &v) {
+        if (v.empty()) return;
+        PDAL_CUDA(cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice, stream_));
+        h2d += (int64_t)(v.size() * sizeof(int));
+    };
+    for (int f = 0; f < 2; ++f)
+        for (int q = 0; q < 2 && flow_smem_[f]; ++q) {
+            Sliced &l = sl_[f][q];
+            const DevMatrix &M = q ? A_ : At_;
+            up(l.desc, l.h.desc);
+            up(l.rl, l.h.rl);
+            up(l.cta, l.cut);
+            k_slice_pack<<<grid_for(32LL * l.h.n), kThreads, 0, stream_>>>(l.h.n, l.desc, l.rl, M.it.d.linfo, S_it_,
+                                                                          M.rp, (const int *)M.ci, l.ci);
+            PDAL_LAUNCH_CHECK();
+        }
+}
+
+/* the equilibrated values in slices, in each precision the solve runs in */
+void CpalSolver::pack_flow() {
+    for (int f = 0; f < 2; ++f)
+        for (int q = 0; q < 2 && flow_smem_[f]; ++q) {
+            const Sliced &l = sl_[f][q];
+            const DevMatrix &M = q ? A_ : At_;
+            const int g = grid_for(32LL * l.h.n);
+            if (f)
+                k_slice_pack<<<g, kThreads, 0, stream_>>>(l.h.n, l.desc, l.rl, M.it.d.linfo, S_it_, M.rp,
+                                                          (const double *)M.v, (double *)l.val);
+            else
+                k_slice_pack<<<g, kThreads, 0, stream_>>>(l.h.n, l.desc, l.rl, M.it.d.linfo, S_it_, M.rp,
+                                                          (const double *)M.v, (float *)l.val);
+            PDAL_LAUNCH_CHECK();
+            launches += 1;
+        }
+}
+
+/* no entry carries a tag (before an estimate, and before the iteration) */
+void CpalSolver::clear_flow() {
+    if (!flow_xt_) return;
+    PDAL_CUDA(cudaMemsetAsync(flow_xt_, 0, sizeof(ulonglong2) * ((size_t)n_ << flow_shift_[0]), stream_));
+    PDAL_CUDA(cudaMemsetAsync(flow_ut_, 0, sizeof(ulonglong2) * ((size_t)m_ << flow_shift_[1]), stream_));
+    PDAL_CUDA(cudaMemsetAsync(flow_sums_, 0, sizeof(ulonglong2) * 32 * (size_t)flow_grid_, stream_));
+    for (int f = 0; f < 2; ++f)
+        for (int q = 0; q < 2 && flow_smem_[f]; ++q)
+            PDAL_CUDA(cudaMemsetAsync(sl_[f][q].part, 0,
+                                      sizeof(ulonglong2) * 8 * (size_t)std::max((q ? A_ : At_).it.hp.npieces, 1),
+                                      stream_));
+}
+
+template <typename T>
+SliceDev<T> CpalSolver::slice_dev(int q) const {
+    const Sliced &l = sl_[sizeof(T) == 8][q];
+    const DevMatrix &M = q ? A_ : At_;
+    return SliceDev<T>{l.desc, l.rl, l.ci, (const T *)l.val, l.cta, M.it.d.linfo, M.rp,
+                       (typename Tagged<T>::Word *)l.part, l.h.n, M.it.d.nlong, S_it_,
+                       O_.persistent_loop == 1};
+}
+
+/* a cooperative launch of one CTA per SM (also inside a stream capture) */
+template <typename... K, typename... A>
+void CpalSolver::launch_coop(void (*kern)(K...), int threads, size_t smem, A... args) {
+    PDAL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFlowSmem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)flow_grid_);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream_;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    PDAL_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+}
+
+/* A device wait that ran out (a staging wait of k_primal_tma, an
+ * exchange of a resident launch) stops the solve (status kStatusDeviceError) and is
  * reported here as an error. */
 void CpalSolver::check_device_error() {
     if (!dev_err_) return;
@@ -810,7 +932,7 @@ void CpalSolver::check_device_error() {
     PDAL_CUDA(cudaMemcpyAsync(&e, dev_err_, sizeof(int), cudaMemcpyDeviceToHost, stream_));
     PDAL_CUDA(cudaStreamSynchronize(stream_));
     if (e == 1) throw Error("a staged copy of the primal product did not complete in time; the solve was stopped");
-    if (e) throw Error("a grid barrier of the persistent loop did not complete in time; the solve was stopped");
+    if (e) throw Error("an exchange between the blocks of a resident launch did not complete in time; the solve was stopped");
 }
 
 void CpalSolver::upload() {
@@ -920,6 +1042,7 @@ void CpalSolver::upload() {
         longs(m_, prob_->constraint_matrix_row_pointers, eq_long_h_[0]);
         longs(n_, At_host_.rp.data(), eq_long_h_[1]);
     }
+    plan_flow();
     const double t_alloc = now_sec();
     upload_plan_sec = t_alloc - t_up;
     arena_.begin_measure();
@@ -963,6 +1086,7 @@ void CpalSolver::upload() {
     upload_plan(At_.it);
     upload_plan(A_.ev);
     upload_plan(At_.ev);
+    upload_flow();
     if (use_panels_) {
         const size_t len = (size_t)pan_host_.len, hp = (size_t)pan_host_.H * pan_host_.P;
         up(sh_r1_, sh_r1_h.data(), sh_r1_h.size() * sizeof(int));
@@ -1039,6 +1163,11 @@ void CpalSolver::upload() {
         PDAL_CUDA(cudaMemsetAsync(y00_, 0, std::max<size_t>(m, 1) * sizeof(double), stream_));
     PDAL_CUDA(cudaStreamSynchronize(stream_));
     At_host_ = HostCsr(); /* host transpose no longer needed */
+    for (auto &f : sl_)
+        for (auto &l : f) {
+            l.h.desc = std::vector<int>();
+            l.h.rl = std::vector<int>();
+        }
     pan_host_.pmap = decltype(pan_host_.pmap)();
     pan_host_.off = decltype(pan_host_.off)();
     upload_sec = now_sec() - t_up;
@@ -1080,6 +1209,19 @@ static void launch_pdl(void (*kern)(KArgs...), int grid, cudaStream_t stream, Ar
     PDAL_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
 }
 
+template <typename T>
+FlowPowerArgs<T> CpalSolver::power_args() {
+    FlowPowerArgs<T> L{};
+    L.at = slice_dev<T>(0);
+    L.a = slice_dev<T>(1);
+    L.dt = tagged_x<T>();
+    L.vt = tagged_u<T>();
+    L.sums = flow_sums_;
+    L.ps = ps_;
+    L.guard = guard();
+    return L;
+}
+
 void CpalSolver::power_iteration() {
     PowerState h{};
     h.max_iter = P_.sv_max_iter;
@@ -1110,6 +1252,30 @@ void CpalSolver::power_iteration() {
         k_power_start<double><<<1, kThreads, 0, stream_>>>(m_, tmp_m_, ps_);
     PDAL_LAUNCH_CHECK();
     launches += 1;
+    if (h.max_iter > 0 && O_.persistent_loop != 1 && flow_smem_[f32 ? 0 : 1] > 0) {
+        /* m-sized buffers the iteration has not started to use */
+        clear_flow();
+        const int steps = std::min(h.max_iter, INT32_MAX - 8);
+        auto run = [&](auto args, auto kern, size_t smem) {
+            using T = std::remove_pointer_t<decltype(args.v0)>;
+            args.v0 = (T *)tmp_m_;
+            T *hist[4] = {(T *)tmp_m2_, (T *)tmp_m_, (T *)v64_.y, (T *)v64_.yh};
+            for (int q = 0; q < 4; ++q) args.hist[q] = hist[q];
+            launch_coop(kern, (kFlowWarps + 1) * 32, smem, args, steps);
+        };
+        if (f32)
+            run(power_args<float>(), k_power_flow<float>, flow_smem_[0]);
+        else
+            run(power_args<double>(), k_power_flow<double>, flow_smem_[1]);
+        launches += 1;
+        PDAL_CUDA(cudaMemcpyAsync(h_ps_, ps_, sizeof(PowerState), cudaMemcpyDeviceToHost, stream_));
+        d2h += sizeof(PowerState);
+        check_device_error(); /* waits for the stream */
+        power_iters = h_ps_->iters;
+        const double smax = std::sqrt(h_ps_->s2);
+        host_state.lambda_est = smax * smax;
+        return;
+    }
     const int gres = grid_for(m_);
     const int steps_per_graph = 16;
     cudaGraphExec_t exec = nullptr;
@@ -1366,6 +1532,7 @@ void CpalSolver::setup_device() {
         PDAL_LAUNCH_CHECK();
         launches += 2;
     }
+    pack_flow();
     /* the long rows' values in panel order, in each precision the
      * iteration runs in */
     if (use_panels_) {
@@ -1405,6 +1572,7 @@ void CpalSolver::setup_device() {
     } else {
         power_iteration();
     }
+    clear_flow();
     s.lambda_est = host_state.lambda_est;
     power_sec = now_sec() - t_pow;
     s.pw = P_.bound_objective_rescaling ? 1.0 : (cp_.obj_norm + 1.0) / (cp_.bnd_norm + 1.0);
@@ -1540,61 +1708,30 @@ const HalpernWf *weights<float>(const HalpernW *, const HalpernWf *w32) {
     return w32;
 }
 
+/* F iterations in one launch */
 template <typename T>
-void CpalSolver::launch_loop(int max_blocks) {
+void CpalSolver::launch_flow(int F) {
     auto &v = vecs<T>();
-    LoopArgs<T> L{};
-    L.at_it = At_.it.d;
-    L.a_it = A_.it.d;
-    L.at_ev = At_.ev.d;
-    L.a_ev = A_.ev.d;
-    if (m_ == 0) {
-        L.a_it.nblocks = 0;
-        L.a_ev.nblocks = 0;
-    }
-    L.at_rp = At_.rp;
-    L.at_ci = At_.ci;
-    L.a_rp = A_.rp;
-    L.a_ci = A_.ci;
-    L.at_val = matvals<T>(At_.v, At_.vf);
-    L.a_val = matvals<T>(A_.v, A_.vf);
-    L.at_v64 = At_.v;
-    L.a_v64 = A_.v;
+    FlowArgs<T> L{};
+    L.at = slice_dev<T>(0);
+    L.a = slice_dev<T>(1);
     L.pa = PrimalArgs<T>{v.x, v.xbar, v.xh, v.lam, anchor<T>(x0_, x0f_), v.c, v.vlb, v.vub};
     L.da = DualArgs<T>{v.y, v.yh, v.ybar, v.ax, v.u, anchor<T>(y0_, y0f_), anchor<T>(ax0_, ax0f_), v.clb, v.cub};
     L.gat = beta_on_ ? v.u : v.y;
-    L.ra = EvalRowArgs<T>{v.xh, v.xbar, v.yh, v.ybar, x0_, y0_, ax0_, clb_, cub_, clbf_, cubf_, rsc_, phat_, part_row_,
-                          A_.ev.d.nblocks, v.x, v.y, v.ax};
-    L.ca = EvalColArgs<T>{v.xh, v.xbar, v.yh, v.ybar, v.lam, x0_, c_, dsc_, part_col_, At_.ev.d.nblocks, v.x, v.y, y0_};
+    L.xt = tagged_x<T>();
+    L.ut = tagged_u<T>();
     L.st = st_;
-    L.p = cp_;
-    L.wt = wt_;
-    L.wtf = wtf_;
-    L.nrow_slots = m_ > 0 ? A_.ev.d.nblocks + A_.ev.d.nlong : 0;
-    L.ncol_slots = At_.ev.d.nblocks + At_.ev.d.nlong;
-    L.n = n_;
-    L.m = m_;
-    const bool f32 = std::is_same<T, float>::value;
-    L.x0 = x0_;
-    L.y0 = y0_;
-    L.ax0 = ax0_;
-    L.x0f = f32 ? x0f_ : nullptr;
-    L.y0f = f32 ? y0f_ : nullptr;
-    L.ax0f = f32 ? ax0f_ : nullptr;
-    L.phat = phat_;
-    L.bar = loop_bar_;
-    L.spin_limit = 1LL << 22; /* polls of an L2 round trip each: a barrier wait gives up after about 2 s */
-    L.max_blocks = max_blocks;
-    L.err = dev_err_;
-    void *args[] = {(void *)&L};
-    const int grid = loop_grid_[f32 ? 0 : 1];
-    /* the barrier counter counts up from zero within a launch */
-    PDAL_CUDA(cudaMemsetAsync(loop_bar_, 0, sizeof(LoopBar), stream_));
-    PDAL_WITH_S_LOOP(S_it_, {
-        const void *kern = beta_on_ ? (const void *)k_cpal_loop<T, SL, SL, true> : (const void *)k_cpal_loop<T, SL, SL, false>;
-        PDAL_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kThreads), args, 0, stream_));
-    });
-    launches += 1;
+    L.wt = weights<T>(wt_, wtf_);
+    L.F = F;
+    L.guard = guard();
+    L.bar = flow_bar_;
+    const size_t smem = flow_smem_[sizeof(T) == 8];
+    if (flow_form<T>() == Flow::barrier) {
+        PDAL_CUDA(cudaMemsetAsync(flow_bar_, 0, sizeof(unsigned), stream_));
+        launch_coop(beta_on_ ? k_flow<T, true, true> : k_flow<T, false, true>, kFlowWarps * 32, smem, L);
+    } else {
+        launch_coop(beta_on_ ? k_flow<T, true, false> : k_flow<T, false, false>, kFlowWarps * 32, smem, L);
+    }
 }
 
 template <typename T>
@@ -1852,7 +1989,9 @@ void CpalSolver::capture_block(cudaGraphExec_t &exec, int F) {
     PDAL_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     for (int g = 0; g < G; ++g) {
         if (timing && g == 0) PDAL_CUDA(cudaEventRecordWithFlags(ev_[3], stream_, cudaEventRecordExternal));
-        for (int i = 1; i <= F; ++i) {
+        const bool resident = flow_form<T>() != Flow::launches;
+        if (resident) launch_flow<T>(F);
+        for (int i = 1; i <= F && !resident; ++i) {
             /* one non-major iteration (F-1 >= 2) is bracketed by events */
             if (timing && g == 0 && i == F - 1) {
                 PDAL_CUDA(cudaEventRecordWithFlags(ev_[0], stream_, cudaEventRecordExternal));
@@ -2156,39 +2295,25 @@ void CpalSolver::run_loop() {
     PDAL_LAUNCH_CHECK();
     launches += 1;
     const int fp32_cap = O_.fp32_max_iterations;
-    setup_loop();
     for (;;) {
-        if (use_loop_) {
-            /* evaluation blocks on the device until a termination, the end
-             * of the FP32 phase or this many blocks (the host then checks
-             * its wall-clock guard and prints the verbose line) */
-            int chunk = (P_.verbose || (fp32_phase_ && fp32_cap >= 0)) ? 1 : 50;
-            /* the launch's barrier counter (blocks x barriers) stays below 2^31 */
-            const long long per = (2LL * F + 3) * std::max(loop_grid_[0], loop_grid_[1]);
-            chunk = (int)std::max(1LL, std::min<long long>(chunk, (1LL << 31) / std::max(per, 1LL)));
-            if (fp32_phase_)
-                launch_loop<float>(chunk);
-            else
-                launch_loop<double>(chunk);
+        const int Fb = h_st_->F; /* this block's length (the dynamic evaluation frequency may shorten it) */
+        const bool res = (fp32_phase_ ? flow_form<float>() : flow_form<double>()) != Flow::launches;
+        const int64_t per_block = (res ? 1 : (int64_t)iter_launches() * Fb) + (m_ > 0 ? 4 : 3) +
+                                  (cp_.infeas ? (m_ > 0 ? 2 : 1) : 0);
+        cudaGraphExec_t *exec;
+        if (fp32_phase_) {
+            exec = &exec32_[beta_on_ ? 1 : 0][Fb != F ? 1 : 0];
+            if (!*exec) capture_block<float>(*exec, Fb);
         } else {
-            const int Fb = h_st_->F; /* this block's length (the dynamic evaluation frequency may shorten it) */
-            const int64_t per_block = (int64_t)iter_launches() * Fb + (m_ > 0 ? 4 : 3) +
-                                      (cp_.infeas ? (m_ > 0 ? 2 : 1) : 0);
-            cudaGraphExec_t *exec;
-            if (fp32_phase_) {
-                exec = &exec32_[beta_on_ ? 1 : 0][Fb != F ? 1 : 0];
-                if (!*exec) capture_block<float>(*exec, Fb);
-            } else {
-                exec = &exec64_[beta_on_ ? 1 : 0][Fb != F ? 1 : 0];
-                if (!*exec) capture_block<double>(*exec, Fb);
-            }
-            PDAL_CUDA(cudaGraphLaunch(*exec, stream_));
-            launches += (per_block + ((fp32_phase_ ? hot_in<float>() : hot_in<double>()) ? 1 : 0)) * G;
+            exec = &exec64_[beta_on_ ? 1 : 0][Fb != F ? 1 : 0];
+            if (!*exec) capture_block<double>(*exec, Fb);
         }
+        PDAL_CUDA(cudaGraphLaunch(*exec, stream_));
+        launches += (per_block + ((fp32_phase_ ? hot_in<float>() : hot_in<double>()) ? 1 : 0)) * G;
         PDAL_CUDA(cudaMemcpyAsync(h_st_, st_, sizeof(CpalState), cudaMemcpyDeviceToHost, stream_));
         d2h += sizeof(CpalState);
         PDAL_CUDA(cudaStreamSynchronize(stream_));
-        if (!use_loop_ && O_.timing && F >= 3 && ev_[0]) {
+        if (O_.timing && F >= 3 && ev_[0]) {
             float a = 0, b = 0, c = 0;
             PDAL_CUDA(cudaEventElapsedTime(&a, ev_[0], ev_[1]));
             PDAL_CUDA(cudaEventElapsedTime(&b, ev_[1], ev_[2]));
