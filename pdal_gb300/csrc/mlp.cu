@@ -3,9 +3,8 @@
  * with the library's own CUDA kernels (sm_103a).
  *
  * The network is three layers of width 256.  Training runs in FP32 on
- * register-tiled SIMT GEMMs (64 x 64 output tile per block, 4 x 4 per
- * thread) with fused bias / ReLU epilogues, plus elementwise backward, Adam
- * and reduction kernels.  BF16 inference runs its three products on the
+ * register-tiled SIMT GEMMs with the bias, ReLU, loss, ReLU gradient and Adam
+ * update in their epilogues.  BF16 inference runs its three products on the
  * tensor cores (mma.sync m16n8k16, FP32 accumulation, k_gemm_bf16_tc), each
  * layer writing the next one's BF16 operand.  All reductions run in a fixed
  * order, so a training run and a prediction are reproducible bit for bit.
@@ -29,85 +28,372 @@ namespace {
 
 thread_local std::string g_mlp_error;
 
-constexpr int TM = 64, TN = 64, TK = 16, GT = 256;
+constexpr int GT = 256;
 
-__device__ __forceinline__ float to_f(float v) { return v; }
+__device__ __forceinline__ uint32_t smem_addr(const void *p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+/* 16 bytes, the first `bytes` of them from src and zeros behind */
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(bytes) : "memory");
+}
+/* four bytes, zeros when !in */
+__device__ __forceinline__ void cp_async4(void *dst, const void *src, bool in) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(in ? 4 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 
-/* C[m, n] = sum_k A(m, k) B(k, n) (+ C) (+ bias[n]) (ReLU); A(m, k) is
- * A[k*lda + m] when TA, else A[m*lda + k]; B(k, n) is B[n*ldb + k] when TB,
- * else B[k*ldb + n]. */
-template <typename TI, bool TA, bool TB>
-__global__ void __launch_bounds__(GT) k_gemm(int M, int N, int K, const TI *__restrict__ A, long long lda,
-                                             const TI *__restrict__ B, long long ldb, float *C, long long ldc,
-                                             const float *__restrict__ bias, int relu, int accumulate) {
-    __shared__ float As[TK][TM + 4];
-    __shared__ float Bs[TK][TN + 4];
+/* ---- FP32 products ---------------------------------------------------- */
+/*
+ * C[M][N] = sum_k A(m, k) B(k, n): every element one chain of FP32 fused
+ * multiply-adds in k order, whatever the tile.  The operands' elements are
+ *   A(m, k)  A[row(m) * lda + k], or with TA A[row(k) * lda + m]
+ *   B(k, n)  B[k * ldb + n],      or with TB B[n * ldb + k]
+ * where row(i) = rows ? rows[i] : i picks the rows of a mini-batch in place.
+ *
+ * The network's products are small and long (layer 1 at a batch of 128: 128 x
+ * 256 outputs of 3,280 terms), so what bounds them is how many SMs have a
+ * tile and how far ahead of the chain the loads run: tiles of 64, 32 or 16
+ * squared, the largest that gives every SM one, fed by a ring of stages of 32
+ * or 64 terms (cp.async, 16 bytes where an operand's rows are aligned and run
+ * along its stage's rows, else 4: the output layer's rows have odd lengths).
+ * A is kept [m][k] in shared memory (one 128-bit load per row and four
+ * terms), or [k][m] with TA.
+ * Measured (3,280 -> 256 -> 256 -> 1,681, batch 128): a training step 98 us,
+ * against 1,070 us with 64 x 64 tiles only, whose layer 1 ran in 8 blocks, and
+ * separate gather, bias, ReLU, loss, column-sum and Adam passes.  Layer 1 takes
+ * 34 us of it and is bound by the issue of one warp per scheduler along its
+ * 3,280-term chains; splitting the sums over clusters was 7 us a step slower
+ * end to end and changes the rounding, which Adam's first steps amplify.
+ */
+struct GemmOp {
+    int M, N, K;
+    const float *A, *B;
+    long long lda, ldb;
+    const int *rows;
+};
+
+template <int BT, bool TA>
+struct Tile {
+    static constexpr int TK = BT == 16 ? 64 : 32;
+    static constexpr int RM = BT == 64 ? 4 : BT == 32 ? 2 : 1; /* a thread's rows and columns */
+    static constexpr int RN = BT == 64 ? 4 : 2;
+    static constexpr int NT = BT * BT / (RM * RN);
+    static constexpr int STAGES = BT == 64 ? 3 : 4;
+    static constexpr int LA = TA ? BT + 4 : TK + 4, NA = TA ? TK : BT; /* A's row length and rows */
+    static constexpr int LB = BT + 4;
+    struct Stage {
+        float a[NA][LA];
+        float b[TK][LB];
+    };
+    static constexpr size_t BYTES = sizeof(Stage) * STAGES;
+};
+
+/* The thread's RM x RN outputs of the tile at (m0, n0); elements outside the
+ * matrices count as zeros.  With `colsum`, thread n < BT also adds the B
+ * elements of column n in k order. */
+template <int BT, bool TA, bool TB>
+__device__ __forceinline__ void tile_sum(const GemmOp &g, int m0, int n0, unsigned char *smem,
+                                         float (&acc)[Tile<BT, TA>::RM][Tile<BT, TA>::RN], float *colsum) {
+    using T = Tile<BT, TA>;
+    constexpr int TK = T::TK, RM = T::RM, RN = T::RN, NT = T::NT, ST = T::STAGES;
+    auto *st = reinterpret_cast<typename T::Stage *>(smem);
+    const int tid = threadIdx.x, tx = tid % (BT / RN), ty = tid / (BT / RN);
+#pragma unroll
+    for (int i = 0; i < RM; ++i)
+#pragma unroll
+        for (int j = 0; j < RN; ++j) acc[i][j] = 0.f;
+    const int steps = (g.K + TK - 1) / TK;
+    constexpr int LD = BT * TK / NT; /* elements of each operand a thread copies per stage */
+    static_assert(LD % 4 == 0 && NT % (TK / 4) == 0 && NT % (BT / 4) == 0, "whole vectors, one column per thread");
+    /* neighbouring threads take neighbouring addresses; whole 16-byte vectors
+     * where every row starts on one */
+    const bool va = g.lda % 4 == 0 && ((uintptr_t)g.A & 15) == 0;
+    const bool vb = !TB && g.ldb % 4 == 0 && ((uintptr_t)g.B & 15) == 0;
+    constexpr int FA = TA ? BT : TK; /* A's contiguous index and the others */
+    /* without TA the rows a thread copies are the same in every stage: found
+     * once, so that no copy waits for a row number */
+    const float *arow[TA ? 1 : LD];
+    if (!TA) {
+#pragma unroll
+        for (int q = 0; q < LD; ++q) {
+            const int e = va ? 4 * (tid + (q < LD / 4 ? q : 0) * NT) : tid + q * NT, m = m0 + e / FA;
+            arow[TA ? 0 : q] =
+                m < g.M ? g.A + (long long)(g.rows ? g.rows[m] : m) * g.lda + e % FA : nullptr;
+        }
+    }
+    auto copy = [&](int step) {
+        typename T::Stage &s = st[step % ST];
+        const int k0 = step * TK;
+        if (va) {
+#pragma unroll
+            for (int q = 0; q < LD / 4; ++q) {
+                const int e = 4 * (tid + q * NT), f = e % FA, r = e / FA;
+                const int m = m0 + f, k = k0 + (TA ? r : f);
+                int bytes = max(0, min(16, 4 * (TA ? g.M - m : g.K - k)));
+                if (TA ? k >= g.K : !arow[TA ? 0 : q]) bytes = 0;
+                const float *src = g.A;
+                if (bytes) src = TA ? g.A + (long long)(g.rows ? g.rows[k] : k) * g.lda + m : arow[TA ? 0 : q] + k0;
+                cp_async16(&s.a[r][f], src, bytes);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < LD; ++q) {
+                const int e = tid + q * NT, f = e % FA, r = e / FA;
+                const int m = m0 + f, k = k0 + (TA ? r : f);
+                const bool in = k < g.K && (TA ? m < g.M : arow[TA ? 0 : q] != nullptr);
+                const float *src = g.A;
+                if (in) src = TA ? g.A + (long long)(g.rows ? g.rows[k] : k) * g.lda + m : arow[TA ? 0 : q] + k0;
+                cp_async4(&s.a[r][f], src, in);
+            }
+        }
+        if (vb) {
+#pragma unroll
+            for (int q = 0; q < LD / 4; ++q) {
+                const int e = 4 * (tid + q * NT), n = n0 + e % BT, k = k0 + e / BT;
+                const int bytes = k < g.K ? max(0, min(16, 4 * (g.N - n))) : 0;
+                cp_async16(&s.b[e / BT][e % BT], bytes ? g.B + (long long)k * g.ldb + n : g.B, bytes);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < LD; ++q) {
+                const int e = tid + q * NT;
+                const int nn = TB ? e / TK : e % BT, kb = TB ? e % TK : e / BT, n = n0 + nn, k = k0 + kb;
+                const bool in = n < g.N && k < g.K;
+                cp_async4(&s.b[kb][nn],
+                          in ? g.B + (TB ? (long long)n * g.ldb + k : (long long)k * g.ldb + n) : g.B, in);
+            }
+        }
+    };
+#pragma unroll
+    for (int q = 0; q < ST - 1; ++q) {
+        if (q < steps) copy(q);
+        cp_async_commit();
+    }
+    for (int t = 0; t < steps; ++t) {
+        cp_async_wait<ST - 2>();
+        __syncthreads(); /* stage t has landed, stage t - 1 is free */
+        if (t + ST - 1 < steps) copy(t + ST - 1);
+        cp_async_commit();
+        const typename T::Stage &s = st[t % ST];
+        /* four terms at a time, the next four loaded before these are used */
+        float a[2][RM][4], b[2][4][RN];
+        auto fetch = [&](int kk, float (&fa)[RM][4], float (&fb)[4][RN]) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (RN == 4) {
+                    const float4 v = *reinterpret_cast<const float4 *>(&s.b[kk + q][tx * RN]);
+                    fb[q][0] = v.x;
+                    fb[q][1] = v.y;
+                    fb[q][RN - 2] = v.z;
+                    fb[q][RN - 1] = v.w;
+                } else {
+                    const float2 v = *reinterpret_cast<const float2 *>(&s.b[kk + q][tx * RN]);
+                    fb[q][0] = v.x;
+                    fb[q][1] = v.y;
+                }
+            }
+            if (TA) {
+                static_assert(!TA || RM == 4, "one 128-bit load per term");
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float4 v = *reinterpret_cast<const float4 *>(&s.a[TA ? kk + q : 0][TA ? ty * RM : 0]);
+                    fa[0][q] = v.x;
+                    fa[RM > 1 ? 1 : 0][q] = v.y;
+                    fa[RM > 2 ? 2 : 0][q] = v.z;
+                    fa[RM > 3 ? 3 : 0][q] = v.w;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < RM; ++i) {
+                    const float4 v = *reinterpret_cast<const float4 *>(&s.a[TA ? 0 : ty * RM + i][TA ? 0 : kk]);
+                    fa[i][0] = v.x;
+                    fa[i][1] = v.y;
+                    fa[i][2] = v.z;
+                    fa[i][3] = v.w;
+                }
+            }
+        };
+        fetch(0, a[0], b[0]);
+#pragma unroll
+        for (int kk = 0; kk < TK; kk += 4) {
+            const int c = (kk >> 2) & 1;
+            if (kk + 4 < TK) fetch(kk + 4, a[c ^ 1], b[c ^ 1]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int i = 0; i < RM; ++i)
+#pragma unroll
+                    for (int j = 0; j < RN; ++j) acc[i][j] = fmaf(a[c][i][q], b[c][q][j], acc[i][j]);
+        }
+        if (colsum && tid < BT)
+#pragma unroll
+            for (int kk = 0; kk < TK; ++kk) *colsum += s.b[kk][tid];
+    }
+    cp_async_wait<0>();
+}
+
+/* what becomes of a finished element v of C */
+enum class Finish {
+    bias_relu, /* C = max(v + bias, 0) */
+    bias,      /* C = v + bias */
+    mask,      /* C = H > 0 ? v : 0 (the ReLU's gradient) */
+    mse        /* P = v + bias: C = scale * (P - Y), the block's sum of (P - Y)^2 in FP64 */
+};
+struct GemmOut {
+    float *C;
+    const float *bias, *H, *Y;
+    const int *rows; /* rows of Y */
+    float scale;
+    double *loss; /* one per block */
+};
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <int BT, bool TB, Finish F>
+__global__ void __launch_bounds__(Tile<BT, false>::NT) k_gemm(GemmOp g, GemmOut o) {
+    using T = Tile<BT, false>;
+    extern __shared__ __align__(16) unsigned char gemm_smem[];
+    __shared__ double sb[T::NT / 32];
+    pdl_wait();
+    const int m0 = blockIdx.y * BT, n0 = blockIdx.x * BT;
+    float acc[T::RM][T::RN];
+    tile_sum<BT, false, TB>(g, m0, n0, gemm_smem, acc, nullptr);
+    const int tx = threadIdx.x % (BT / T::RN), ty = threadIdx.x / (BT / T::RN);
+    double loss = 0.0;
+#pragma unroll
+    for (int i = 0; i < T::RM; ++i)
+#pragma unroll
+        for (int j = 0; j < T::RN; ++j) {
+            const int m = m0 + ty * T::RM + i, n = n0 + tx * T::RN + j;
+            if (m >= g.M || n >= g.N) continue;
+            const float v = acc[i][j];
+            float *c = o.C + (size_t)m * g.N + n;
+            if (F == Finish::bias_relu) {
+                *c = fmaxf(v + o.bias[n], 0.f);
+            } else if (F == Finish::bias) {
+                *c = v + o.bias[n];
+            } else if (F == Finish::mask) {
+                *c = o.H[(size_t)m * g.N + n] > 0.f ? v : 0.f;
+            } else {
+                const float d = (v + o.bias[n]) - o.Y[(size_t)(o.rows ? o.rows[m] : m) * g.N + n];
+                if (o.C) *c = o.scale * d;
+                loss += (double)d * (double)d;
+            }
+        }
+    if (F == Finish::mse) {
+        for (int q = 16; q > 0; q >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, q);
+        if ((threadIdx.x & 31) == 0) sb[threadIdx.x >> 5] = loss;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double t = 0.0;
+            for (int w = 0; w < T::NT / 32; ++w) t += sb[w];
+            o.loss[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = t;
+        }
+    }
+}
+
+/* The weight gradients dW = A^T dZ and bias gradients (the column sums of dZ,
+ * in row order) of the three layers in one launch; each element is stored, or
+ * goes straight into its Adam update, so that a training step writes no
+ * gradient.  The last block adds the batch's loss to `loss_sum`. */
+struct LayerGrad {
+    GemmOp g; /* M x N = the weight's shape, K = rows of the batch */
+    size_t w, b; /* offsets of the weight and the bias in the parameter vector */
+    int tiles_n, first; /* tiles along N, first block */
+};
+struct AdamArgs {
+    float *p, *m, *v, *grad; /* grad: store the gradient instead of updating */
+    float lr, b1, b2, eps, bc1, bc2;
+};
+struct WeightArgs {
+    LayerGrad l[3];
+    AdamArgs adam;
+    const double *loss;
+    int nloss;
+    double inv_count, *loss_sum;
+};
+
+__global__ void __launch_bounds__(GT, 3) k_weights(WeightArgs W) {
+    using T = Tile<64, true>;
+    static_assert(T::NT == GT, "one thread shape for the tiles and the loss");
+    extern __shared__ __align__(16) unsigned char gemm_smem[];
+    pdl_wait();
+    if (blockIdx.x + 1 == gridDim.x) {
+        __shared__ double sb[GT / 32];
+        double t = 0.0;
+        for (int i = threadIdx.x; i < W.nloss; i += GT) t += W.loss[i];
+        for (int q = 16; q > 0; q >>= 1) t += __shfl_xor_sync(0xffffffffu, t, q);
+        if ((threadIdx.x & 31) == 0) sb[threadIdx.x >> 5] = t;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double s = 0.0;
+            for (int w = 0; w < GT / 32; ++w) s += sb[w];
+            *W.loss_sum += s * W.inv_count;
+        }
+        return;
+    }
+    const int li = (int)blockIdx.x >= W.l[2].first ? 2 : (int)blockIdx.x >= W.l[1].first ? 1 : 0;
+    const LayerGrad &l = W.l[li];
+    const int t = blockIdx.x - l.first, m0 = t / l.tiles_n * 64, n0 = t % l.tiles_n * 64;
+    float acc[T::RM][T::RN], col = 0.f;
+    tile_sum<64, true, false>(l.g, m0, n0, gemm_smem, acc, m0 == 0 ? &col : nullptr);
+    const AdamArgs &A = W.adam;
+    auto update = [&](size_t at, float g, float p, float m, float v) {
+        const float mi = A.b1 * m + (1.f - A.b1) * g;
+        const float vi = A.b2 * v + (1.f - A.b2) * g * g;
+        A.m[at] = mi;
+        A.v[at] = vi;
+        A.p[at] = p - A.lr * (mi / A.bc1) / (sqrtf(vi / A.bc2) + A.eps);
+    };
+    /* through shared memory, so that a warp updates neighbouring elements */
+    float(*out)[64] = reinterpret_cast<float(*)[64]>(gemm_smem);
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    float acc[4][4];
+    __syncthreads();
 #pragma unroll
     for (int i = 0; i < 4; ++i)
+        *reinterpret_cast<float4 *>(&out[ty * 4 + i][tx * 4]) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    __syncthreads();
+    const int n = n0 + (threadIdx.x & 63);
+    if (n >= l.g.N) return;
+    /* eight elements' moments loaded before any is used */
+    constexpr int U = 8;
+    for (int r0 = threadIdx.x >> 6; r0 < 64; r0 += 4 * U) {
+        float p[U], m[U], v[U];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    for (int k0 = 0; k0 < K; k0 += TK) {
-        for (int e = threadIdx.x; e < TM * TK; e += GT) {
-            int mm, kk;
-            if (TA) {
-                kk = e / TM;
-                mm = e % TM;
-            } else {
-                mm = e / TK;
-                kk = e % TK;
+        for (int u = 0; u < U; ++u) {
+            const size_t at = l.w + (size_t)(m0 + r0 + 4 * u) * l.g.N + n;
+            if (!A.grad && m0 + r0 + 4 * u < l.g.M) {
+                p[u] = A.p[at];
+                m[u] = A.m[at];
+                v[u] = A.v[at];
             }
-            const int gm = m0 + mm, gk = k0 + kk;
-            float v = 0.f;
-            if (gm < M && gk < K) v = to_f(TA ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk]);
-            As[kk][mm] = v;
         }
-        for (int e = threadIdx.x; e < TN * TK; e += GT) {
-            int nn, kk;
-            if (TB) {
-                nn = e / TK;
-                kk = e % TK;
-            } else {
-                kk = e / TN;
-                nn = e % TN;
-            }
-            const int gn = n0 + nn, gk = k0 + kk;
-            float v = 0.f;
-            if (gn < N && gk < K) v = to_f(TB ? B[(size_t)gn * ldb + gk] : B[(size_t)gk * ldb + gn]);
-            Bs[kk][nn] = v;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int r = r0 + 4 * u;
+            if (m0 + r >= l.g.M) continue;
+            const size_t at = l.w + (size_t)(m0 + r) * l.g.N + n;
+            if (A.grad)
+                A.grad[at] = out[r][n - n0];
+            else
+                update(at, out[r][n - n0], p[u], m[u], v[u]);
         }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < TK; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int gm = m0 + ty * 4 + i;
-        if (gm >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int gn = n0 + tx * 4 + j;
-            if (gn >= N) continue;
-            float v = acc[i][j];
-            float *c = C + (size_t)gm * ldc + gn;
-            if (accumulate) v += *c;
-            if (bias) v += bias[gn];
-            if (relu) v = fmaxf(v, 0.f);
-            *c = v;
-        }
+    if (m0 == 0 && threadIdx.x < 64) {
+        const size_t at = l.b + n;
+        if (A.grad)
+            A.grad[at] = col;
+        else
+            update(at, col, A.p[at], A.m[at], A.v[at]);
     }
 }
 
@@ -123,18 +409,15 @@ __global__ void __launch_bounds__(GT) k_gemm(int M, int N, int K, const TI *__re
  * order, so the result does not depend on the split's timing. */
 constexpr int TCM = 64, TCN = 64, TCK = 32, TCT = 128;
 
-__device__ __forceinline__ uint32_t tc_smem(const void *p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
 __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void *p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(tc_smem(p)));
+                 : "r"(smem_addr(p)));
 }
 __device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const void *p) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(tc_smem(p)));
+                 : "r"(smem_addr(p)));
 }
 __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile(
@@ -143,15 +426,6 @@ __device__ __forceinline__ void mma_bf16_16816(float (&d)[4], const uint32_t (&a
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc_smem(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
 struct TcSmem {
     __nv_bfloat16 a[2][TCM][TCK + 8]; /* rows of 80 bytes: ldmatrix rows fall in distinct banks */
     __nv_bfloat16 b[2][TCK][TCN + 8]; /* rows of 144 bytes */
@@ -257,61 +531,6 @@ __global__ void k_tc_finish(const float *__restrict__ part, int Z, int M, int N,
         if (relu) v = fmaxf(v, 0.f);
         if (C) C[t] = v;
         if (Cb) Cb[t] = __float2bfloat16(v);
-    }
-}
-
-__global__ void k_gather_rows(float *dst, const float *__restrict__ src, const int *__restrict__ idx, int rows,
-                              long long cols) {
-    const size_t total = (size_t)rows * cols;
-    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = t / cols, c = t % cols;
-        dst[t] = src[(size_t)idx[r] * cols + c];
-    }
-}
-
-/* db[n] = sum over rows of dY[:, n] (fixed row order) */
-__global__ void k_colsum(const float *__restrict__ dY, int M, int N, float *db) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    float s = 0.f;
-    for (int m = 0; m < M; ++m) s += dY[(size_t)m * N + n];
-    db[n] = s;
-}
-
-__global__ void k_relu_bwd(float *dH, const float *__restrict__ H, size_t count) {
-    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < count; t += (size_t)gridDim.x * blockDim.x)
-        if (!(H[t] > 0.f)) dH[t] = 0.f;
-}
-
-/* dP = scale * (P - Y); per-block partial sums of (P - Y)^2 in FP64 */
-__global__ void __launch_bounds__(GT) k_mse(const float *__restrict__ P, const float *__restrict__ Y, float *dP,
-                                            size_t count, float scale, double *part) {
-    __shared__ double sb[GT / 32];
-    double s = 0.0;
-    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < count; t += (size_t)gridDim.x * blockDim.x) {
-        const float d = P[t] - Y[t];
-        if (dP) dP[t] = scale * d;
-        s += (double)d * (double)d;
-    }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) sb[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < GT / 32; ++w) t += sb[w];
-        part[blockIdx.x] = t;
-    }
-}
-
-__global__ void k_adam(float *p, const float *__restrict__ g, float *m, float *v, size_t count, float lr, float b1,
-                       float b2, float eps, float bc1, float bc2) {
-    for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < count; t += (size_t)gridDim.x * blockDim.x) {
-        const float gi = g[t];
-        const float mi = b1 * m[t] + (1.f - b1) * gi;
-        const float vi = b2 * v[t] + (1.f - b2) * gi * gi;
-        m[t] = mi;
-        v[t] = vi;
-        p[t] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
     }
 }
 
@@ -423,12 +642,40 @@ __global__ void __launch_bounds__(GT) k_tr_kkt(int S, int D, const double *__res
 
 int grid1(size_t count) { return (int)std::min<size_t>((count + GT - 1) / GT, 152 * 16); }
 
-template <typename TI, bool TA, bool TB>
-void gemm(cudaStream_t s, int M, int N, int K, const TI *A, long long lda, const TI *B, long long ldb, float *C,
-          long long ldc, const float *bias, bool relu, bool accumulate) {
-    if (M <= 0 || N <= 0) return;
-    dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM);
-    k_gemm<TI, TA, TB><<<grid, GT, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, relu ? 1 : 0, accumulate ? 1 : 0);
+/* a launch that is prepared while the kernel before it finishes (every kernel
+ * of the network's products begins with griddepcontrol.wait) */
+template <typename... K, typename... A>
+void launch(void (*kern)(K...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+    if (smem > 48 * 1024)
+        PDAL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    PDAL_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+}
+
+/* returns the number of blocks (the losses of Finish::mse) */
+template <int BT, bool TB, Finish F>
+int gemm_tiles(cudaStream_t s, const GemmOp &g, const GemmOut &o) {
+    using T = Tile<BT, false>;
+    const dim3 grid((g.N + BT - 1) / BT, (g.M + BT - 1) / BT);
+    launch(k_gemm<BT, TB, F>, grid, T::NT, T::BYTES, s, g, o);
+    return (int)(grid.x * grid.y);
+}
+template <bool TB, Finish F>
+int gemm(cudaStream_t s, int sms, const GemmOp &g, const GemmOut &o) {
+    if (g.M <= 0 || g.N <= 0) return 0;
+    auto tiles = [&](long long bt) { return ((g.N + bt - 1) / bt) * ((g.M + bt - 1) / bt); };
+    if (tiles(64) >= sms) return gemm_tiles<64, TB, F>(s, g, o);
+    if (tiles(32) >= sms) return gemm_tiles<32, TB, F>(s, g, o);
+    return gemm_tiles<16, TB, F>(s, g, o);
 }
 
 template <typename T>
@@ -483,15 +730,20 @@ struct Mlp {
     DevBuf<float> P, G, Ma, Va;
     DevBuf<float> Xb, Yb, H1, H2, Yp, dY, dH1, dH2;
     DevBuf<int> idx;
-    DevBuf<double> part;
+    DevBuf<double> part; /* loss sums of the blocks, then the epoch's loss */
+    int sms = 0;
     DevBuf<float> Xd, Yd;
     DevBuf<__nv_bfloat16> Pb, Xbb, H1b, H2b;
+    DevBuf<double> warm[9]; /* instances, results and statistics of a warm-start call */
     DevBuf<float> Tp; /* split-K slices of the tensor-core products */
     int ndata = 0;
     long long adam_t = 0;
 
     Mlp(int in_, int h_, int out_, unsigned seed, int dev) : in(in_), h(h_), out(out_), device(dev) {
         if (device >= 0) PDAL_CUDA(cudaSetDevice(device));
+        int current = 0;
+        PDAL_CUDA(cudaGetDevice(&current));
+        PDAL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, current));
         oW1 = 0;
         ob1 = oW1 + (size_t)in * h;
         oW2 = ob1 + h;
@@ -522,17 +774,20 @@ struct Mlp {
         if (s) cudaStreamDestroy(s);
     }
 
-    void buffers(int B) {
-        Xb.ensure((size_t)B * in);
-        Yb.ensure((size_t)B * out);
+    /* activations of B rows; with `train` also the gradients */
+    void buffers(int B, bool train) {
         H1.ensure((size_t)B * h);
         H2.ensure((size_t)B * h);
-        Yp.ensure((size_t)B * out);
+        if (!train) {
+            Yp.ensure((size_t)B * out);
+            return;
+        }
         dY.ensure((size_t)B * out);
         dH1.ensure((size_t)B * h);
         dH2.ensure((size_t)B * h);
-        part.ensure((size_t)152 * 16);
+        part.ensure((size_t)((out + 15) / 16) * ((B + 15) / 16) + 1);
     }
+    double *loss_sum() const { return part.p + part.n - 1; }
 
     /* inference of B rows of X (device, FP32) into Yp: FP32 SIMT, or BF16
      * operands on the tensor cores (the weights' BF16 copy made by
@@ -558,44 +813,74 @@ struct Mlp {
         gemm_tc(s, B, out, h, H2b.p, h, W3, out, Yp.p, nullptr, b3, false, Tp);
     }
 
+    /* the two hidden layers of B rows of X (device; row i is rows[i]) */
+    void hidden(int B, const float *X, const int *rows) {
+        GemmOut o{};
+        o.C = H1.p;
+        o.bias = P.p + ob1;
+        gemm<false, Finish::bias_relu>(s, sms, GemmOp{B, h, in, X, P.p + oW1, in, h, rows}, o);
+        o.C = H2.p;
+        o.bias = P.p + ob2;
+        gemm<false, Finish::bias_relu>(s, sms, GemmOp{B, h, h, H1.p, P.p + oW2, h, h, nullptr}, o);
+    }
     /* forward of B rows of X (device) into Yp */
     void forward(int B, const float *X) {
-        const float *W1 = P.p + oW1, *b1 = P.p + ob1, *W2 = P.p + oW2, *b2 = P.p + ob2, *W3 = P.p + oW3,
-                    *b3 = P.p + ob3;
-        gemm<float, false, false>(s, B, h, in, X, in, W1, h, H1.p, h, b1, true, false);
-        gemm<float, false, false>(s, B, h, h, H1.p, h, W2, h, H2.p, h, b2, true, false);
-        gemm<float, false, false>(s, B, out, h, H2.p, h, W3, out, Yp.p, out, b3, false, false);
+        hidden(B, X, nullptr);
+        GemmOut o{};
+        o.C = Yp.p;
+        o.bias = P.p + ob3;
+        gemm<false, Finish::bias>(s, sms, GemmOp{B, out, h, H2.p, P.p + oW3, h, out, nullptr}, o);
     }
 
-    /* loss of B rows against Y (device); gradient into G when grad */
-    double loss_backward(int B, const float *X, const float *Y, bool grad) {
+    /* One batch: rows[0..B) (or the first B) of X and Y, their mean squared
+     * error added to loss_sum(), the gradient into A.grad or the Adam update.
+     * Without `back` the loss alone. */
+    void step(int B, const float *X, const float *Y, const int *rows, const AdamArgs &A, bool back) {
         const size_t cnt = (size_t)B * out;
-        const int g = grid1(cnt);
-        k_mse<<<g, GT, 0, s>>>(Yp.p, Y, grad ? dY.p : nullptr, cnt, 2.0f / (float)cnt, part.p);
-        std::vector<double> hp(g);
-        if (grad) {
-            const float *W2 = P.p + oW2, *W3 = P.p + oW3;
-            /* layer 3 */
-            gemm<float, true, false>(s, h, out, B, H2.p, h, dY.p, out, G.p + oW3, out, nullptr, false, false);
-            k_colsum<<<(out + GT - 1) / GT, GT, 0, s>>>(dY.p, B, out, G.p + ob3);
-            gemm<float, false, true>(s, B, h, out, dY.p, out, W3, out, dH2.p, h, nullptr, false, false);
-            k_relu_bwd<<<grid1((size_t)B * h), GT, 0, s>>>(dH2.p, H2.p, (size_t)B * h);
-            /* layer 2 */
-            gemm<float, true, false>(s, h, h, B, H1.p, h, dH2.p, h, G.p + oW2, h, nullptr, false, false);
-            k_colsum<<<(h + GT - 1) / GT, GT, 0, s>>>(dH2.p, B, h, G.p + ob2);
-            gemm<float, false, true>(s, B, h, h, dH2.p, h, W2, h, dH1.p, h, nullptr, false, false);
-            k_relu_bwd<<<grid1((size_t)B * h), GT, 0, s>>>(dH1.p, H1.p, (size_t)B * h);
-            /* layer 1 */
-            gemm<float, true, false>(s, in, h, B, X, in, dH1.p, h, G.p + oW1, h, nullptr, false, false);
-            k_colsum<<<(h + GT - 1) / GT, GT, 0, s>>>(dH1.p, B, h, G.p + ob1);
+        hidden(B, X, rows);
+        GemmOut o{};
+        o.C = back ? dY.p : nullptr;
+        o.bias = P.p + ob3;
+        o.Y = Y;
+        o.rows = rows;
+        o.scale = 2.0f / (float)cnt;
+        o.loss = part.p;
+        WeightArgs W{};
+        W.nloss = gemm<false, Finish::mse>(s, sms, GemmOp{B, out, h, H2.p, P.p + oW3, h, out, nullptr}, o);
+        W.loss = part.p;
+        W.inv_count = 1.0 / (double)cnt;
+        W.loss_sum = loss_sum();
+        W.adam = A;
+        int blocks = 0;
+        if (back) {
+            GemmOut d{};
+            d.C = dH2.p;
+            d.H = H2.p;
+            gemm<true, Finish::mask>(s, sms, GemmOp{B, h, out, dY.p, P.p + oW3, out, out, nullptr}, d);
+            d.C = dH1.p;
+            d.H = H1.p;
+            gemm<true, Finish::mask>(s, sms, GemmOp{B, h, h, dH2.p, P.p + oW2, h, h, nullptr}, d);
+            /* the largest first */
+            const GemmOp g[3] = {{in, h, B, X, dH1.p, in, h, rows},
+                                 {h, out, B, H2.p, dY.p, h, out, nullptr},
+                                 {h, h, B, H1.p, dH2.p, h, h, nullptr}};
+            const size_t ow[3] = {oW1, oW3, oW2}, ob[3] = {ob1, ob3, ob2};
+            for (int q = 0; q < 3; ++q) {
+                const int tn = (g[q].N + 63) / 64, tm = (g[q].M + 63) / 64;
+                W.l[q] = LayerGrad{g[q], ow[q], ob[q], tn, blocks};
+                blocks += tn * tm;
+            }
         }
-        PDAL_CUDA(cudaMemcpyAsync(hp.data(), part.p, sizeof(double) * g, cudaMemcpyDeviceToHost, s));
+        launch(k_weights, dim3(blocks + 1), GT, Tile<64, true>::BYTES, s, W);
+    }
+    double read_loss() {
+        double t = 0.0;
+        PDAL_CUDA(cudaMemcpyAsync(&t, loss_sum(), sizeof(double), cudaMemcpyDeviceToHost, s));
         PDAL_CUDA(cudaStreamSynchronize(s));
         PDAL_CUDA(cudaGetLastError());
-        double t = 0.0;
-        for (double v : hp) t += v;
-        return t / (double)cnt;
+        return t;
     }
+    void clear_loss() { PDAL_CUDA(cudaMemsetAsync(loss_sum(), 0, sizeof(double), s)); }
 };
 
 } // namespace pdal
@@ -681,35 +966,27 @@ double pdal_mlp_train(pdal_mlp_t *h, int epochs, int batch, float lr, unsigned s
         pdal::Mlp &m = *h->m;
         const int n = m.ndata;
         const int B = std::min(batch, n);
-        m.buffers(B);
+        m.buffers(B, true);
         m.idx.ensure(n);
         std::vector<int> perm(n);
         std::iota(perm.begin(), perm.end(), 0);
         std::mt19937 gen(seed);
         double last = 0.0;
-        const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+        pdal::AdamArgs A{m.P.p, m.Ma.p, m.Va.p, nullptr, lr, 0.9f, 0.999f, 1e-8f, 0.f, 0.f};
         for (int ep = 0; ep < epochs; ++ep) {
             std::shuffle(perm.begin(), perm.end(), gen);
             PDAL_CUDA(cudaMemcpyAsync(m.idx.p, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice, m.s));
-            double sum = 0.0;
+            m.clear_loss();
             int batches = 0;
             for (int b0 = 0; b0 + B <= n; b0 += B) {
-                pdal::k_gather_rows<<<pdal::grid1((size_t)B * m.in), pdal::GT, 0, m.s>>>(m.Xb.p, m.Xd.p, m.idx.p + b0,
-                                                                                        B, m.in);
-                pdal::k_gather_rows<<<pdal::grid1((size_t)B * m.out), pdal::GT, 0, m.s>>>(
-                    m.Yb.p, m.Yd.p, m.idx.p + b0, B, m.out);
-                m.forward(B, m.Xb.p);
-                sum += m.loss_backward(B, m.Xb.p, m.Yb.p, true);
                 ++batches;
                 ++m.adam_t;
-                const float bc1 = 1.f - std::pow(b1, (float)m.adam_t), bc2 = 1.f - std::pow(b2, (float)m.adam_t);
-                pdal::k_adam<<<pdal::grid1(m.np), pdal::GT, 0, m.s>>>(m.P.p, m.G.p, m.Ma.p, m.Va.p, m.np, lr, b1, b2,
-                                                                      eps, bc1, bc2);
+                A.bc1 = 1.f - std::pow(A.b1, (float)m.adam_t);
+                A.bc2 = 1.f - std::pow(A.b2, (float)m.adam_t);
+                m.step(B, m.Xd.p, m.Yd.p, m.idx.p + b0, A, true);
             }
-            last = batches ? sum / batches : 0.0;
+            if (ep + 1 == epochs) last = batches ? m.read_loss() / batches : 0.0;
         }
-        PDAL_CUDA(cudaStreamSynchronize(m.s));
-        PDAL_CUDA(cudaGetLastError());
         return last;
     } catch (const std::exception &e) {
         return fail(e.what());
@@ -720,11 +997,16 @@ double pdal_mlp_loss_grad(pdal_mlp_t *h, int n, const float *X, const float *Y, 
     if (!h || n <= 0 || !X || !Y) return fail("pdal_mlp_loss_grad: invalid arguments");
     try {
         pdal::Mlp &m = *h->m;
-        m.buffers(n);
+        m.buffers(n, true);
+        m.Xb.ensure((size_t)n * m.in);
+        m.Yb.ensure((size_t)n * m.out);
         PDAL_CUDA(cudaMemcpyAsync(m.Xb.p, X, (size_t)n * m.in * 4, cudaMemcpyHostToDevice, m.s));
         PDAL_CUDA(cudaMemcpyAsync(m.Yb.p, Y, (size_t)n * m.out * 4, cudaMemcpyHostToDevice, m.s));
-        m.forward(n, m.Xb.p);
-        const double loss = m.loss_backward(n, m.Xb.p, m.Yb.p, grad != nullptr);
+        m.clear_loss();
+        pdal::AdamArgs A{};
+        A.grad = m.G.p;
+        m.step(n, m.Xb.p, m.Yb.p, nullptr, A, grad != nullptr);
+        const double loss = m.read_loss();
         if (grad) PDAL_CUDA(cudaMemcpy(grad, m.G.p, m.np * 4, cudaMemcpyDeviceToHost));
         return loss;
     } catch (const std::exception &e) {
@@ -737,7 +1019,8 @@ int pdal_mlp_predict(pdal_mlp_t *h, int n, const float *X, float *Y, int bf16) {
     try {
         pdal::Mlp &m = *h->m;
         const int chunk = std::min(n, 1024);
-        m.buffers(chunk);
+        m.buffers(chunk, false);
+        m.Xb.ensure((size_t)chunk * m.in);
         if (bf16) m.prepare_bf16(chunk);
         for (int r0 = 0; r0 < n; r0 += chunk) {
             const int B = std::min(chunk, n - r0);
@@ -768,9 +1051,10 @@ int pdal_transport_warm_start(pdal_mlp_t *h, int S, int D, int count, const doub
         if (m.in != 2 * n + mm || m.out != n + mm + 1)
             return fail("pdal_transport_warm_start: the network's sizes do not match the S x D family");
         const int chunk = std::min(count, 1024);
-        m.buffers(chunk);
+        m.buffers(chunk, false);
+        m.Xb.ensure((size_t)chunk * m.in);
         if (bf16) m.prepare_bf16(chunk);
-        pdal::DevBuf<double> dc, du, db, dx, dy, ds, dk0, dk1, st;
+        auto &[dc, du, db, dx, dy, ds, dk0, dk1, st] = m.warm;
         dc.ensure((size_t)chunk * n);
         du.ensure((size_t)chunk * n);
         db.ensure((size_t)chunk * mm);
