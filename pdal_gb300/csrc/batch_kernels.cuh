@@ -137,7 +137,7 @@ struct EvalRowsB : Base {
 /* ------------------------------------------------------------------ setup */
 
 /* Ruiz (mode 0) or Pock-Chambolle (mode 1) pass, the block-level form of
- * k_row_scale / k_scale_matrix / k_scale_vectors (same operation order: the
+ * k_equil_pass / k_equil_vectors (same operation order: the
  * Pock-Chambolle sums in row order in one lane, as the reference adds them). */
 __device__ void blk_scale_pass(const BInst &I, int mode, double deg_rows, double deg_cols) {
     auto row_scale = [&](int nr, const int *rp, const double *val, double deg, double *scale, double *cum) {

@@ -1537,8 +1537,6 @@ __global__ void k_convert(const A *__restrict__ src, B *dst, int len) {
 /* setup: equilibration (LP/CP_AL/src/preconditioner.cu)               */
 /* ------------------------------------------------------------------ */
 
-/* warp per row: s = clamp_sqrt(max |a| or sum |a|^deg), cum *= s
- * (preconditioner.cu:532-550, 634-667). mode 0 = abs max, 1 = power sum. */
 /* ------------------------------------------------------------------ */
 /* the transpose A^T built on the device                               */
 /* ------------------------------------------------------------------ */
@@ -1652,68 +1650,179 @@ static __global__ void k_hot_indices(long long nnz, const int *__restrict__ ci, 
     }
 }
 
-/* Equilibration passes over the rows of a CSR matrix.  Rows of at most
- * kEqShort nonzeros (nearly all rows of a sparse LP) run one thread per row;
- * the longer rows, listed once at upload (`lrows`), run one warp per row in
- * the same launch.  (A warp per row for every row left 31 lanes idle on the
- * one-entry rows of a power-law LP and made each pass latency-bound.) */
-__device__ __forceinline__ double row_scale_term(double v, int mode, double deg) {
-    v = fabs(v);
-    if (!isfinite(v)) v = 0.0;
-    if (mode == 0) return v;
+/* One equilibration pass over a row block of a CSR matrix: the previous pass's
+ * scales applied to its values, and the next pass's row statistic of the
+ * scaled values (Ruiz: max |a|, LP/CP_AL/src/preconditioner.cu:273-378;
+ * Pock-Chambolle: sum |a|^deg, 600-657), so that a pass reads and writes the
+ * matrix once.  The values stream through shared memory nonzero by nonzero
+ * (whole lines, the products in full warps) and are then reduced row by row:
+ * maxima as integers, since the bits of non-negative doubles order as the
+ * numbers do and the FP64 pipe would bound them; sums in row order in one
+ * thread, as the reference adds them.  A long row's pieces leave their
+ * statistics in plan.lpart, added by the block that comes last in piece order.
+ * Measured (10M nonzeros, 8M of them in 760 long rows): 3.0 ms a pass with a
+ * thread per row, its 32 lanes in 32 lines, and statistic, matrix and vectors
+ * apart; 0.35 ms so. */
+enum : int { kStatNone = 0, kStatMax = 1, kStatSum = 2 };
+
+__device__ __forceinline__ unsigned long long abs_bits(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+    return b < 0x7ff0000000000000ull ? b : 0ull; /* not finite: 0 */
+}
+__device__ __forceinline__ double row_scale_term(double v, double deg) {
+    v = __longlong_as_double((long long)abs_bits(v));
     if (deg == 2.0) return v * v;
     if (deg == 1.0) return v;
     if (deg == 0.5) return sqrt(v);
     return pow(v, deg);
 }
 
-__device__ __forceinline__ void row_scale_store(int row, double acc, double *scale, double *cum, double *inv) {
-    const double s = (acc < 1e-12) ? 1.0 : sqrt(acc);
-    cum[row] *= s;
-    scale[row] = s;
-    inv[row] = 1.0 / s;
-}
-
-/* Ruiz (mode 0: max |a|) or Pock-Chambolle (mode 1: sum |a|^deg) row scale
- * (LP/CP_AL/src/preconditioner.cu:273-378, 600-657).  The sums run in row
- * order in one thread, as the reference's kernel adds them (a long row too);
- * the maxima of the long rows take a warp (the order does not matter). */
-static __global__ void k_row_scale(int nr, const int *__restrict__ rp, const double *__restrict__ val, int mode, double deg,
-                            double *scale, double *cum, double *inv, const int *__restrict__ lrows, int nlong) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
-    for (int row = t; row < nr; row += nt) {
-        const int k0 = rp[row], k1 = rp[row + 1];
-        if (k1 - k0 > kEqShort) continue;
-        double acc = 0.0;
-        for (int k = k0; k < k1; ++k) {
-            const double pv = row_scale_term(val[k], mode, deg);
-            acc = mode == 0 ? fmax(acc, pv) : acc + pv;
-        }
-        row_scale_store(row, acc, scale, cum, inv);
+template <int S>
+__global__ void __launch_bounds__(kThreads) k_equil_pass(RowPlanDev plan, const int *__restrict__ rp,
+                                                         const int *__restrict__ ci, double *val,
+                                                         const double *__restrict__ inv_row,
+                                                         const double *__restrict__ inv_col, int apply, int stat,
+                                                         double deg, double *out) {
+    constexpr int NT = kThreads, NW = NT / 32, U = 4;
+    __shared__ double sv[S];
+    __shared__ unsigned short srow[S];
+    __shared__ int srp[kMaxRowsPerBlock + 1];
+    __shared__ double red[NW];
+    __shared__ int slast;
+    const int4 d = plan.desc[blockIdx.x];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool piece = d.y < d.x;
+    const int lid = ~d.y, row0 = d.x, nrows = piece ? 1 : d.y - d.x, cnt = d.w - d.z;
+    if (!piece) {
+        for (int t = tid; t <= nrows; t += NT) srp[t] = rp[row0 + t] - d.z;
+        __syncthreads();
+        if (apply)
+            for (int r = warp; r < nrows; r += NW)
+                for (int k = srp[r] + lane; k < srp[r + 1]; k += 32) srow[k] = (unsigned short)r;
+        __syncthreads();
     }
-    if (mode != 0) {
-        for (int q = t; q < nlong; q += nt) {
-            const int row = lrows[q];
-            double acc = 0.0;
-            for (int k = rp[row]; k < rp[row + 1]; ++k) acc += row_scale_term(val[k], mode, deg);
-            row_scale_store(row, acc, scale, cum, inv);
+    unsigned long long mx = 0; /* of a piece */
+    double sum = 0.0;
+    for (int k0 = tid; k0 < cnt; k0 += U * NT) {
+        double v[U], p[U];
+        int c[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + u * NT;
+            if (k < cnt) {
+                v[u] = val[d.z + k];
+                if (apply) c[u] = ci[d.z + k];
+            }
+        }
+        if (apply) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (k0 + u * NT < cnt)
+                    p[u] = inv_row[piece ? row0 : row0 + srow[k0 + u * NT]] * inv_col[c[u]];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (k0 + u * NT < cnt) {
+                    v[u] *= p[u];
+                    val[d.z + k0 + u * NT] = v[u];
+                }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (k0 + u * NT < cnt) {
+                if (!piece)
+                    sv[k0 + u * NT] = v[u];
+                else if (stat == kStatMax)
+                    mx = max(mx, abs_bits(v[u]));
+                else if (stat == kStatSum)
+                    sum += row_scale_term(v[u], deg);
+            }
+    }
+    if (stat == kStatNone) return;
+    if (!piece) {
+        __syncthreads();
+        if (stat == kStatSum) {
+            for (int r = tid; r < nrows; r += NT) {
+                double acc = 0.0;
+                for (int k = srp[r]; k < srp[r + 1]; ++k) acc += row_scale_term(sv[k], deg);
+                out[row0 + r] = acc;
+            }
+            return;
+        }
+        int g = 32;
+        while (g > 1 && g * nrows > NT) g >>= 1;
+        for (int r0 = 0; r0 < nrows; r0 += NT / g) {
+            const int r = r0 + tid / g;
+            unsigned long long m = 0;
+            if (r < nrows)
+                for (int k = srp[r] + (tid & (g - 1)); k < srp[r + 1]; k += g) m = max(m, abs_bits(sv[k]));
+            for (int o = g >> 1; o > 0; o >>= 1) m = max(m, __shfl_down_sync(0xffffffffu, m, o, g));
+            if (r < nrows && (tid & (g - 1)) == 0) out[row0 + r] = __longlong_as_double((long long)m);
         }
         return;
     }
-    const int lane = threadIdx.x & 31;
-    for (int q = t >> 5; q < nlong; q += nt >> 5) {
-        const int row = lrows[q];
-        double acc = 0.0;
-        for (int k = rp[row] + lane; k < rp[row + 1]; k += 32) acc = fmax(acc, row_scale_term(val[k], 0, deg));
-        acc = warp_max(acc);
-        if (lane == 0) row_scale_store(row, acc, scale, cum, inv);
+    const int4 li = plan.linfo[lid];
+    double mine = stat == kStatSum ? warp_sum(sum) : 0.0;
+    if (stat == kStatMax) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        mine = __longlong_as_double((long long)mx);
+    }
+    if (lane == 0) red[warp] = mine;
+    __syncthreads();
+    if (tid == 0) {
+        double t = 0.0;
+        for (int w = 0; w < NW; ++w) t = stat == kStatSum ? t + red[w] : fmax(t, red[w]);
+        plan.lpart[(size_t)(li.z + (d.z - li.w) / S) * kLongStride] = t;
+        __threadfence();
+        slast = atomicAdd(&plan.lcount[lid], 1u) == (unsigned)(li.y - 1);
+    }
+    __syncthreads();
+    if (!slast || tid != 0) return;
+    __threadfence();
+    double t = 0.0;
+    for (int q = 0; q < li.y; ++q) {
+        const double v = __ldcg(&plan.lpart[(size_t)(li.z + q) * kLongStride]);
+        t = stat == kStatSum ? t + v : fmax(t, v);
+    }
+    plan.lcount[lid] = 0u;
+    out[li.x] = t;
+}
+
+/* The scales of a pass from its statistics, s = sqrt(stat) (1 below 1e-12),
+ * their reciprocals for the matrices, and the vectors
+ * (LP/CP_AL/src/preconditioner.cu:476-512). */
+__device__ __forceinline__ double equil_scale(double stat) { return stat < 1e-12 ? 1.0 : sqrt(stat); }
+static __global__ void k_equil_vectors(int n, int m, const double *__restrict__ dstat, const double *__restrict__ rstat,
+                                       double *dcum, double *rcum, double *dinv, double *rinv, double *c, double *vlb,
+                                       double *vub, double *x0, double *clb, double *cub, double *y0) {
+    const int total = n > m ? n : m;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+        if (t < n) {
+            const double s = equil_scale(dstat[t]), inv = 1.0 / s;
+            dcum[t] *= s;
+            dinv[t] = inv;
+            c[t] *= inv;
+            vlb[t] *= s;
+            vub[t] *= s;
+            x0[t] *= s;
+        }
+        if (t < m) {
+            const double s = equil_scale(rstat[t]), inv = 1.0 / s;
+            rcum[t] *= s;
+            rinv[t] = inv;
+            clb[t] *= inv;
+            cub[t] *= inv;
+            y0[t] *= s;
+        }
     }
 }
 
+static __global__ void k_fill(int len, double v, double *dst) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < len; i += gridDim.x * blockDim.x) dst[i] = v;
+}
+
 /* A values *= (1/d[j]) * (1/r[i]); rows of this matrix are scaled by
- * row_is_var ? d : r (preconditioner.cu:514-530).  The reciprocals come from
- * k_row_scale (the same 1/s, computed once per row instead of once per
- * nonzero: the FP64 divisions dominated this kernel on GB300's FP64 pipe). */
+ * row_is_var ? d : r (preconditioner.cu:514-530): the Curtis-Reid scales. */
 static __global__ void k_scale_matrix(int nr, const int *__restrict__ rp, const int *__restrict__ ci, double *val,
                                const double *__restrict__ inv_rowscale, const double *__restrict__ inv_colscale,
                                int row_is_var, const int *__restrict__ lrows, int nlong) {
@@ -1819,27 +1928,6 @@ static __global__ void k_scale_vectors_inv(int n, int m, const double *__restric
             clb[t] *= rinv[t];
             cub[t] *= rinv[t];
             y0[t] *= r[t];
-        }
-    }
-}
-
-/* preconditioner.cu:476-512 */
-static __global__ void k_scale_vectors(int n, int m, const double *__restrict__ d, const double *__restrict__ r, double *c,
-                                double *vlb, double *vub, double *x0, double *clb, double *cub, double *y0) {
-    const int total = n > m ? n : m;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-        if (t < n) {
-            const double dj = d[t], inv = 1.0 / d[t];
-            c[t] *= inv;
-            vlb[t] *= dj;
-            vub[t] *= dj;
-            x0[t] *= dj;
-        }
-        if (t < m) {
-            const double inv = 1.0 / r[t], ei = r[t];
-            clb[t] *= inv;
-            cub[t] *= inv;
-            y0[t] *= ei;
         }
     }
 }

@@ -1437,27 +1437,25 @@ void CpalSolver::setup_device() {
     /* equilibration: LP/CP_AL/src/preconditioner.cu:379-475 */
     const int gn = grid_for(n), gm = grid_for(m);
     const int gwr_m = grid_for((long long)m * 32), gwr_n = grid_for((long long)n * 32);
-    std::vector<double> ones_n(n, 1.0), ones_m(m, 1.0);
-    PDAL_CUDA(cudaMemcpyAsync(dsc_, ones_n.data(), n * sizeof(double), cudaMemcpyHostToDevice, stream_));
-    if (m) PDAL_CUDA(cudaMemcpyAsync(rsc_, ones_m.data(), m * sizeof(double), cudaMemcpyHostToDevice, stream_));
+    k_fill<<<gn, kThreads, 0, stream_>>>(n_, 1.0, dsc_);
+    if (m) k_fill<<<gm, kThreads, 0, stream_>>>(m_, 1.0, rsc_);
     double *rstep = tmp_m_, *dstep = tmp_n_;
     /* reciprocal scales: an m- and an n-sized buffer the iteration has not
      * started to use (x_bar is cleared before the first iteration) */
     double *rinv = tmp_m2_, *dinv = v64_.xbar;
     const int nla = (int)eq_long_h_[0].size(), nlt = (int)eq_long_h_[1].size();
     const int geq_m = grid_for(std::max<long long>(m, 32LL * nla)), geq_n = grid_for(std::max<long long>(n, 32LL * nlt));
-    auto scale_pass = [&](int mode, double deg_rows, double deg_cols) {
-        if (m)
-            k_row_scale<<<geq_m, kThreads, 0, stream_>>>(m_, A_.rp, A_.v, mode, deg_rows, rstep, rsc_, rinv, eq_long_[0],
-                                                         nla);
-        k_row_scale<<<geq_n, kThreads, 0, stream_>>>(n_, At_.rp, At_.v, mode, deg_cols, dstep, dsc_, dinv, eq_long_[1],
-                                                     nlt);
-        if (m) k_scale_matrix<<<geq_m, kThreads, 0, stream_>>>(m_, A_.rp, A_.ci, A_.v, rinv, dinv, 0, eq_long_[0], nla);
-        k_scale_matrix<<<geq_n, kThreads, 0, stream_>>>(n_, At_.rp, At_.ci, At_.v, dinv, rinv, 1, eq_long_[1], nlt);
-        k_scale_vectors<<<grid_for(std::max(n, m)), kThreads, 0, stream_>>>(n_, m_, dstep, rstep, c_, vlb_, vub_, x0_,
-                                                                            clb_, cub_, y0_);
+    /* the scales of the pass before applied, the statistics of the next one */
+    auto matrix_pass = [&](int apply, int stat, double deg_rows, double deg_cols) {
+        PDAL_WITH_S(S_it_, {
+            if (m)
+                k_equil_pass<SB><<<A_.it.d.nblocks, kThreads, 0, stream_>>>(A_.it.d, A_.rp, A_.ci, A_.v, rinv, dinv,
+                                                                           apply, stat, deg_rows, rstep);
+            k_equil_pass<SB><<<At_.it.d.nblocks, kThreads, 0, stream_>>>(At_.it.d, At_.rp, At_.ci, At_.v, dinv, rinv,
+                                                                        apply, stat, deg_cols, dstep);
+        });
         PDAL_LAUNCH_CHECK();
-        launches += 5;
+        launches += 2;
     };
     /* Curtis-Reid before Ruiz (LP/CP_AL/src/preconditioner.cu:162-270,
      * 403-425): alternating row / column log-mean passes, then the scales
@@ -1503,8 +1501,20 @@ void CpalSolver::setup_device() {
         PDAL_LAUNCH_CHECK();
         launches += 5;
     }
-    for (int it = 0; it < P_.l_inf_ruiz_iterations; ++it) scale_pass(0, 0.0, 0.0);
-    if (P_.has_pock_chambolle_alpha) scale_pass(1, P_.pock_chambolle_alpha, 2.0 - P_.pock_chambolle_alpha);
+    {
+        const int ruiz = std::max(P_.l_inf_ruiz_iterations, 0), passes = ruiz + (P_.has_pock_chambolle_alpha ? 1 : 0);
+        const double alpha = P_.pock_chambolle_alpha;
+        auto stat_of = [&](int p) { return p >= passes ? kStatNone : p < ruiz ? kStatMax : kStatSum; };
+        if (passes > 0) matrix_pass(0, stat_of(0), alpha, 2.0 - alpha);
+        for (int p = 0; p < passes; ++p) {
+            k_equil_vectors<<<grid_for(std::max(n, m)), kThreads, 0, stream_>>>(n_, m_, dstep, rstep, dsc_, rsc_, dinv,
+                                                                                rinv, c_, vlb_, vub_, x0_, clb_, cub_,
+                                                                                y0_);
+            PDAL_LAUNCH_CHECK();
+            launches += 1;
+            matrix_pass(1, stat_of(p + 1), alpha, 2.0 - alpha);
+        }
+    }
     const int gb = grid_for(std::max(n, m));
     k_boundobj_partials<<<gb, kThreads, 0, stream_>>>(n_, m_, clb_, cub_, c_, part_misc_);
     k_boundobj_finish<<<1, kThreads, 0, stream_>>>(part_misc_, gb, st_, P_.bound_objective_rescaling ? 1 : 0);
