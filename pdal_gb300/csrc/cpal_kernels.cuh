@@ -1659,7 +1659,8 @@ static __global__ void k_hot_indices(long long nnz, const int *__restrict__ ci, 
  * maxima as integers, since the bits of non-negative doubles order as the
  * numbers do and the FP64 pipe would bound them; sums in row order in one
  * thread, as the reference adds them.  A long row's pieces leave their
- * statistics in plan.lpart, added by the block that comes last in piece order.
+ * statistics in plan.lpart, added by the block that comes last in piece order
+ * (sums of the FP64 form: k_equil_long_sums).
  * Measured (10M nonzeros, 8M of them in 760 long rows): 3.0 ms a pass with a
  * thread per row, its 32 lanes in 32 lines, and statistic, matrix and vectors
  * apart; 0.35 ms so. */
@@ -1786,6 +1787,28 @@ __global__ void __launch_bounds__(kThreads) k_equil_pass(RowPlanDev plan, const 
     }
     plan.lcount[lid] = 0u;
     out[li.x] = t;
+}
+
+/* The Pock-Chambolle sums of the rows that k_equil_pass sums in pieces, again in
+ * row order as the reference adds them, a warp per row.  The FP64 form runs in
+ * the reference's arithmetic, and a power-law LP's reduced costs there move by
+ * up to 3e-8 of their rms with this order; one chain of FP64 adds of the longest
+ * row (64 cycles each), once per equilibration. */
+static __global__ void k_equil_long_sums(RowPlanDev plan, const int *__restrict__ rp, const double *__restrict__ val,
+                                         double deg, double *out) {
+    const int lane = threadIdx.x & 31, lid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (lid >= plan.nlong) return;
+    const int row = plan.linfo[lid].x, end = rp[row + 1];
+    double acc = 0.0;
+    int k = rp[row];
+    double next = k + lane < end ? row_scale_term(val[k + lane], deg) : 0.0;
+    for (; k < end; k += 32) {
+        const double t = next;
+        if (k + 32 + lane < end) next = row_scale_term(val[k + 32 + lane], deg);
+        const int n = min(32, end - k);
+        for (int j = 0; j < n; ++j) acc += __shfl_sync(0xffffffffu, t, j);
+    }
+    if (lane == 0) out[row] = acc;
 }
 
 /* The scales of a pass from its statistics, s = sqrt(stat) (1 below 1e-12),

@@ -1454,8 +1454,17 @@ void CpalSolver::setup_device() {
             k_equil_pass<SB><<<At_.it.d.nblocks, kThreads, 0, stream_>>>(At_.it.d, At_.rp, At_.ci, At_.v, dinv, rinv,
                                                                         apply, stat, deg_cols, dstep);
         });
-        PDAL_LAUNCH_CHECK();
         launches += 2;
+        if (stat == kStatSum && !fp32_phase_)
+            for (const DevMatrix *M : {&A_, &At_}) {
+                const RowPlanDev &plan = M->it.d;
+                if (plan.nlong == 0) continue;
+                const bool rows = M == &A_;
+                k_equil_long_sums<<<(plan.nlong + 7) / 8, kThreads, 0, stream_>>>(
+                    plan, M->rp, M->v, rows ? deg_rows : deg_cols, rows ? rstep : dstep);
+                launches += 1;
+            }
+        PDAL_LAUNCH_CHECK();
     };
     /* Curtis-Reid before Ruiz (LP/CP_AL/src/preconditioner.cu:162-270,
      * 403-425): alternating row / column log-mean passes, then the scales
