@@ -209,6 +209,9 @@ class CpalSolver {
     IterVecs<T> &vecs();
     void power_iteration();
     void lanczos();
+    void start_vector(double *v);
+    unsigned *mt_words_ = nullptr;
+    int *mt_count_ = nullptr;
     /* the chosen form estimates sigma_max^2 by Lanczos unless told otherwise */
     bool use_lanczos() const { return m_ > 0 && fp32_phase_ && O_.power_method != 0; }
     void switch_to_fp64();
@@ -263,10 +266,7 @@ class CpalSolver {
     bool fuse_finish_ = false;
     /* the dual step's short-row and panel launches on two streams (forked and
      * joined with events, also inside the captured graphs) */
-    bool dual_fork_ = false;   /* in the FP64 phase */
-    bool dual_fork32_ = false; /* also in the FP32 phase */
-    template <typename T>
-    bool forked() const { return dual_fork_ && (dual_fork32_ || std::is_same<T, double>::value); }
+    bool dual_fork_ = false;
     cudaStream_t side_ = nullptr;
     cudaEvent_t fork_ev_ = nullptr, join_ev_ = nullptr;
     unsigned *pan_cnt_ = nullptr;
@@ -640,6 +640,8 @@ void CpalSolver::alloc_all() {
     if (device_transpose_) at_cursor_ = arena_.take<int>(n + 1);
     if (device_transpose_ && use_hot_) hot_id_d_ = arena_.take<int>(std::max<size_t>(m, 1));
     alloc_flow();
+    mt_words_ = arena_.take<unsigned>(624 * (size_t)mt_twists(m_));
+    mt_count_ = arena_.take<int>(mt_blocks(m_));
     if (use_panels_) {
         const size_t len = (size_t)pan_host_.len, hp = (size_t)pan_host_.H * pan_host_.P;
         const size_t n1 = std::max<size_t>(sh_r1_h.size(), 1), n2 = std::max<size_t>(sh_r2_h.size(), 1),
@@ -1023,9 +1025,8 @@ void CpalSolver::upload() {
             sh_b3_ = blocks((long long)sh_r3_h.size(), kThreads / 32, 152 * 2);
             use_panels_ = pan_host_.H > 0;
             fuse_finish_ = O_.dual_fused_finish == 1;
-            /* measured: the FP64 dual step 0.212 -> 0.200 ms, the FP32 one no faster */
+            /* an iteration of the large LP: FP32 98.9 -> 97 us, FP64 183 -> 178 us */
             dual_fork_ = use_panels_ && !fuse_finish_ && O_.dual_concurrent != 0;
-            dual_fork32_ = dual_fork_ && O_.dual_concurrent == 1;
             if (dual_fork_ && !side_) {
                 PDAL_CUDA(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking));
                 PDAL_CUDA(cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming));
@@ -1222,27 +1223,48 @@ FlowPowerArgs<T> CpalSolver::power_args() {
     return L;
 }
 
+/* The start vector of the sigma_max estimates, std::normal_distribution over
+ * std::mt19937(1) as the reference draws it in a fresh process
+ * (LP/CP_AL/src/utils.cu:27-28, 102-106), on the device (k_mt_*); the launches
+ * draw 1.4 words per word needed on average and a margin of ten deviations. */
+void CpalSolver::start_vector(double *v) {
+    const int blocks = mt_blocks(m_), pairs = 156 * mt_twists(m_);
+    MtSeed seed;
+    seed.x[0] = 1u;
+    for (int i = 1; i < 624; ++i) seed.x[i] = 1812433253u * (seed.x[i - 1] ^ (seed.x[i - 1] >> 30)) + (unsigned)i;
+    k_mt_words<<<1, kMtThreads, 0, stream_>>>(seed, mt_twists(m_), mt_words_);
+    k_mt_count<<<blocks, kThreads, 0, stream_>>>(mt_words_, pairs, mt_count_);
+    k_mt_normals<<<blocks, kThreads, 0, stream_>>>(mt_words_, pairs, mt_count_, m_, v);
+    PDAL_LAUNCH_CHECK();
+    launches += 3;
+}
+
 void CpalSolver::power_iteration() {
     PowerState h{};
     h.max_iter = P_.sv_max_iter;
     h.tol = P_.sv_tol;
     h.done = (h.max_iter <= 0) ? 1 : 0;
-    /* start vector: std::normal_distribution over std::mt19937(1), as the
-     * reference draws it in a fresh process (LP/CP_AL/src/utils.cu:27-28, 102-106) */
-    std::vector<double> v0(m_);
-    std::mt19937 gen(1);
-    std::normal_distribution<double> dist(0.0, 1.0);
-    for (int i = 0; i < m_; ++i) v0[i] = dist(gen);
     /* plain form: FP64 over the evaluation plans; chosen form: FP32 over the
      * iteration plans and the FP32 matrix copies (made before this call) */
     const bool f32 = fp32_phase_;
-    if (f32) {
-        std::vector<float> v0f(v0.begin(), v0.end());
-        PDAL_CUDA(cudaMemcpyAsync(tmp_m_, v0f.data(), sizeof(float) * m_, cudaMemcpyHostToDevice, stream_));
-        h2d += sizeof(float) * m_;
-    } else {
+    const bool flow = h.max_iter > 0 && O_.persistent_loop != 1 && flow_smem_[f32 ? 0 : 1] > 0;
+    std::vector<double> v0;
+    if (!f32 && !flow) {
+        /* the plain form of a large LP keeps the host's logarithm and order of
+         * sums: its power-law LPs amplify one unit in the last place of the
+         * estimate to 1e-7 of the reduced costs */
+        v0.resize(m_);
+        std::mt19937 gen(1);
+        std::normal_distribution<double> dist(0.0, 1.0);
+        for (int i = 0; i < m_; ++i) v0[i] = dist(gen);
         PDAL_CUDA(cudaMemcpyAsync(tmp_m_, v0.data(), sizeof(double) * m_, cudaMemcpyHostToDevice, stream_));
         h2d += sizeof(double) * m_;
+    } else {
+        start_vector(f32 ? tmp_m2_ : tmp_m_);
+        if (f32) {
+            k_convert<double, float><<<grid_for(m_), kThreads, 0, stream_>>>(tmp_m2_, (float *)tmp_m_, m_);
+            launches += 1;
+        }
     }
     *h_ps_ = h;
     PDAL_CUDA(cudaMemcpyAsync(ps_, h_ps_, sizeof(PowerState), cudaMemcpyHostToDevice, stream_));
@@ -1252,7 +1274,7 @@ void CpalSolver::power_iteration() {
         k_power_start<double><<<1, kThreads, 0, stream_>>>(m_, tmp_m_, ps_);
     PDAL_LAUNCH_CHECK();
     launches += 1;
-    if (h.max_iter > 0 && O_.persistent_loop != 1 && flow_smem_[f32 ? 0 : 1] > 0) {
+    if (flow) {
         /* m-sized buffers the iteration has not started to use */
         clear_flow();
         const int steps = std::min(h.max_iter, INT32_MAX - 8);
@@ -1336,12 +1358,7 @@ void CpalSolver::power_iteration() {
  * it stops when that value moves by less than 1e-8 relative over a chunk, at
  * an invariant subspace, or after min(kLanczosMax, sv_max_iter) steps. */
 void CpalSolver::lanczos() {
-    std::vector<double> v0(m_);
-    std::mt19937 gen(1);
-    std::normal_distribution<double> dist(0.0, 1.0);
-    for (int i = 0; i < m_; ++i) v0[i] = dist(gen);
-    PDAL_CUDA(cudaMemcpyAsync(tmp_m_, v0.data(), sizeof(double) * m_, cudaMemcpyHostToDevice, stream_));
-    h2d += sizeof(double) * m_;
+    start_vector(tmp_m_);
     PowerState h{};
     h.inv = 1.0; /* the product kernels scale their input by inv */
     h.max_iter = 1 << 30;
@@ -1351,10 +1368,11 @@ void CpalSolver::lanczos() {
     /* FP32 buffers the iteration has not started to use */
     float *qf = v32_.ybar, *w = v32_.u, *dp = reinterpret_cast<float *>(tmp_n_);
     const LanczosDev lz{lz_alpha_, lz_beta_, lz_j_};
-    k_lz_start<float><<<1, kThreads, 0, stream_>>>(m_, tmp_m_, qf, tmp_m2_);
-    PDAL_LAUNCH_CHECK();
-    launches += 1;
     const int gm = grid_for(m_);
+    k_lz_norm<<<gm, kThreads, 0, stream_>>>(m_, tmp_m_, part_misc_);
+    k_lz_start<float><<<gm, kThreads, 0, stream_>>>(m_, tmp_m_, qf, tmp_m2_, part_misc_, gm);
+    PDAL_LAUNCH_CHECK();
+    launches += 2;
     const int nparts = A_.it.d.nblocks + A_.it.d.nlong;
     cudaGraphExec_t exec = nullptr;
     PDAL_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
@@ -1844,7 +1862,7 @@ void CpalSolver::launch_dual(int koff, bool major, bool timed) {
     }
     const PanelDev<T> pd = panel_dev<T>();
     const size_t psm = panel_smem_bytes<T>(pd.W);
-    if (forked<T>()) {
+    if (dual_fork_) {
         /* the panel partials on the side stream, concurrently with the short
          * rows: both only read x-bar and write disjoint outputs */
         PDAL_CUDA(cudaEventRecord(fork_ev_, stream_));
@@ -1872,7 +1890,7 @@ void CpalSolver::launch_dual(int koff, bool major, bool timed) {
     /* the long rows: panel partials, then one warp per row for the sum and
      * the dual epilogue */
     const int gf = (pd.H * 32 + kThreads - 1) / kThreads;
-    if (forked<T>()) {
+    if (dual_fork_) {
         PDAL_CUDA(cudaStreamWaitEvent(stream_, join_ev_, 0));
         if (major) {
             if (beta_on_)
@@ -2341,7 +2359,7 @@ void CpalSolver::run_loop() {
             sum_ms[ph][0] += a;
             sum_ms[ph][1] += b;
             sum_ms[ph][2] += c;
-            if (use_panels_ && !(fp32_phase_ ? forked<float>() : forked<double>())) {
+            if (use_panels_ && !dual_fork_) {
                 float d = 0, e = 0;
                 PDAL_CUDA(cudaEventElapsedTime(&d, ev_[1], ev_[4]));
                 PDAL_CUDA(cudaEventElapsedTime(&e, ev_[4], ev_[5]));

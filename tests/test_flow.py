@@ -71,3 +71,37 @@ def test_resident_forms_match_the_launches(lp_lib, case, protocol):
         for u, v in ((a.x, b.x), (a.y, b.y), (a.reduced_cost, b.reduced_cost)):
             assert np.linalg.norm(u - v) <= tol * (1 + np.linalg.norm(u))
         assert np.array_equal(b.x, again.x) and np.array_equal(b.y, again.y)
+
+
+def _normals(m):
+    """std::normal_distribution over mt19937(1): Marsaglia's polar method on
+    pairs of 64-bit uniforms, low word first, the second coordinate's variate
+    first."""
+    raw = np.random.MT19937()
+    raw._legacy_seeding(1)
+    w = raw.random_raw(8 * m + 400).astype(np.float64).reshape(-1, 2)
+    u = 2.0 * ((w[:, 0] + w[:, 1] * 2.0**32) / 2.0**64) - 1.0
+    x, y = u[0::2], u[1::2]
+    r2 = x * x + y * y
+    x, y, r2 = (a[(r2 <= 1.0) & (r2 > 0.0)] for a in (x, y, r2))
+    f = np.sqrt(-2.0 * np.log(r2) / r2)
+    return np.stack([y * f, x * f], 1).ravel()[:m]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 2, 3, 1023, 3000, 20001])
+def test_start_vector_of_the_power_iteration(lp_lib, m):
+    """One step from the start vector v, scalings off, A = [I | e_i]: the
+    quotient is 1 + v_i^2 / |v|^2, for the first, a middle and the last i.
+    Rounding: a few eps per variate and sums of m terms in FP64: 1e-12."""
+    v = _normals(m)
+    for i in {0, m // 2, m - 1}:
+        cols = np.concatenate([np.arange(m), [m]])
+        rows = np.concatenate([np.arange(m), [i]])
+        A = sp.csr_matrix((np.ones(m + 1), (rows, cols)), shape=(m, m + 1))
+        d = lp.LPData(np.ones(m + 1), A=A, con_lb=np.zeros(m), con_ub=np.full(m, 5.0), var_lb=np.zeros(m + 1),
+                      var_ub=np.full(m + 1, 4.0))
+        p = {"eps": 1e-14, "iteration_limit": 1, "sv_max_iter": 1, "l_inf_ruiz_iterations": 0,
+             "has_pock_chambolle_alpha": 0}
+        g = lp.solve(d, p, {"precision": "fp64"})
+        assert g.stats["lambda_est"] == pytest.approx(1.0 + v[i] ** 2 / (v @ v), rel=1e-12)
