@@ -189,31 +189,34 @@ struct Cx {
  * returned the count, a reset, a generation word, four fences and polls 64 ns
  * apart.)  A QP of 50,000 variables in FP64, 300 iterations of about five
  * products: 43.0 -> 36.0 ms with the warp-per-term sums of greduce. */
-__device__ bool gsync(Cx &cx) {
-    GridBar *b = cx.P.bar;
+__device__ __forceinline__ bool grid_barrier(GridBar *b, unsigned nb, int extra, long long spin_limit, unsigned &sense,
+                                             int *sok) {
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
-        const unsigned add = blockIdx.x == 0 ? 0x80000000u - (cx.nb + (unsigned)cx.P.bar_extra - 1u) : 1u;
+        const unsigned add = blockIdx.x == 0 ? 0x80000000u - (nb + (unsigned)extra - 1u) : 1u;
         asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(&b->count), "r"(add) : "memory");
         long long spins = 0;
-        while (((ld_acquire(&b->count) ^ cx.sense) & 0x80000000u) == 0) {
+        while (((ld_acquire(&b->count) ^ sense) & 0x80000000u) == 0) {
             ++spins;
             if ((spins & 63) == 0 && *(volatile int *)&b->err) {
                 ok = 0;
                 break;
             }
-            if (spins > cx.P.spin_limit) {
+            if (spins > spin_limit) {
                 atomicExch(&b->err, 1);
                 ok = 0;
                 break;
             }
         }
-        cx.sense ^= 0x80000000u;
-        *cx.sok = ok;
+        sense ^= 0x80000000u;
+        *sok = ok;
     }
     __syncthreads();
-    return *cx.sok != 0;
+    return *sok != 0;
+}
+__device__ bool gsync(Cx &cx) {
+    return grid_barrier(cx.P.bar, cx.nb, cx.P.bar_extra, cx.P.spin_limit, cx.sense, cx.sok);
 }
 
 #define FACP_SYNC(cx)                                                                                                  \

@@ -13,7 +13,7 @@
 #include "../../include/fa_cp.h"
 #include "../../include/fa_cp_gb300.h"
 #include "common.h"
-#include "facp_kernels.cuh"
+#include "facp_power.cuh"
 
 #include <algorithm>
 #include <memory>
@@ -243,6 +243,49 @@ struct DevMat {
     DMat d{};
 };
 
+/* Slices of 32 rows, a lane per row (facp_power.cuh), the rows of a window of
+ * kPowerWindow by length; none when a row is longer than kPowerChain. */
+struct HostPowerMat {
+    std::vector<int> entries, rows; /* pairs: PowerMat's */
+    long long len = 0;
+    int ns = 0;
+    PowerMat d{};
+};
+static void plan_power(int nr, const std::vector<int> &rp, HostPowerMat &M) {
+    M = HostPowerMat{};
+    for (int i = 0; i < nr; ++i)
+        if (rp[i + 1] - rp[i] > kPowerChain) return;
+    M.ns = (nr + 31) / 32;
+    M.entries.resize(2 * (size_t)M.ns);
+    M.rows.resize(64 * (size_t)M.ns);
+    int at[kPowerChain + 2];
+    for (int r0 = 0; r0 < nr; r0 += kPowerWindow) {
+        const int r1 = std::min(r0 + kPowerWindow, nr);
+        std::fill(at, at + kPowerChain + 2, 0);
+        for (int r = r0; r < r1; ++r) at[kPowerChain - (rp[r + 1] - rp[r]) + 1]++;
+        for (int q = 0; q <= kPowerChain; ++q) at[q + 1] += at[q];
+        for (int r = r0; r < r1; ++r) {
+            int *to = &M.rows[2 * (size_t)(r0 + at[kPowerChain - (rp[r + 1] - rp[r])]++)];
+            to[0] = r;
+            to[1] = rp[r + 1] - rp[r];
+        }
+    }
+    for (size_t k = nr; k < 32 * (size_t)M.ns; ++k) {
+        M.rows[2 * k] = -1;
+        M.rows[2 * k + 1] = 0;
+    }
+    for (int s = 0; s < M.ns; ++s) {
+        const int most = M.rows[64 * (size_t)s + 1]; /* a slice's rows are of one window: the first is the longest */
+        M.entries[2 * (size_t)s] = (int)M.len;
+        M.entries[2 * (size_t)s + 1] = most;
+        M.len += 32LL * most;
+        if (M.len > (long long)INT32_MAX - 65536) {
+            M = HostPowerMat{};
+            return;
+        }
+    }
+}
+
 class FacpSolver {
   public:
     FacpSolver(const qp_problem_t *prob, const fa_cp_parameters_t &prm, const fa_cp_gb300_options_t &opt)
@@ -298,12 +341,15 @@ class FacpSolver {
     double transpose_sec_ = 0.0;
     int qtype_ = Q_NONE;
     DevMat M_[NMAT];
+    HostPowerMat pow_a_, pow_at_, pow_q_;
+    void pack_power(HostPowerMat &M, const DMat &d);
+    void launch_power(int mode, double lam_max);
     Arena arena_;
     Prob P_{};
     Ctl ctl_{};
     cudaStream_t stream_ = nullptr;
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
-    int grid_ = 0;
+    int grid_ = 0, sms_ = 1;
     std::vector<double> diag_;
     double qnorm_ = 0.0, nonconvexity_ = 0.0;
     double sv_max_ = 0.0;
@@ -405,6 +451,14 @@ void FacpSolver::prepare() {
         lbase += dm.plan.nlong;
     }
     P_.nlong_total = lbase;
+    /* the power iterations' slices: A and A' together, Q */
+    pow_a_ = pow_at_ = pow_q_ = HostPowerMat{};
+    if (M_[MAT_A].h.nnz() > 0) {
+        plan_power(P.m, M_[MAT_A].h.rp, pow_a_);
+        if (pow_a_.ns > 0) plan_power(P.n, M_[MAT_AT].h.rp, pow_at_);
+        if (pow_at_.ns == 0) pow_a_ = HostPowerMat{};
+    }
+    if (qtype_ == Q_SPARSE) plan_power(P.n, M_[MAT_Q].h.rp, pow_q_);
     P_.bar_extra = std::max(0, o_.barrier_extra_arrivals);
     P_.spin_limit = o_.barrier_spin_limit > 0 ? o_.barrier_spin_limit : kSpinLimit;
 }
@@ -422,6 +476,7 @@ void FacpSolver::upload() {
     int coop = 0, sms = 0;
     PDAL_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     PDAL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    sms_ = sms;
     if (!coop) throw Error("the device does not support cooperative launches");
     int per_sm = 0;
     PDAL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_facp, kThreads, 0));
@@ -467,8 +522,16 @@ void FacpSolver::upload() {
         P_.pv = arena_.take<double>(vec);
         P_.pv2 = arena_.take<double>(vec);
         P_.pv3 = arena_.take<double>(vec);
-        P_.part = arena_.take<double>((size_t)3 * grid_ * kSlot);
+        P_.part = arena_.take<double>((size_t)3 * std::max(grid_, sms_) * kSlot);
         P_.lpart = arena_.take<double>((size_t)3 * nl * kSlot);
+        for (HostPowerMat *M : {&pow_a_, &pow_at_, &pow_q_}) {
+            M->d.ns = M->ns;
+            if (M->ns == 0) continue;
+            M->d.entries = arena_.take<int2>(M->ns);
+            M->d.rows = arena_.take<int2>(32 * (size_t)M->ns);
+            M->d.ci = arena_.take<int>(std::max<size_t>(M->len, 1));
+            M->d.v = arena_.take<double>(std::max<size_t>(M->len, 1));
+        }
         P_.bar = arena_.take<GridBar>(1);
         P_.ctl = arena_.take<Ctl>(1);
         P_.f = SegV<float>{};
@@ -582,6 +645,59 @@ void FacpSolver::read_ctl() {
     if (ctl_.status != 0) throw Error("the persistent kernel gave up waiting at a grid barrier");
 }
 
+void FacpSolver::pack_power(HostPowerMat &M, const DMat &d) {
+    PDAL_CUDA(cudaMemcpyAsync((void *)M.d.entries, M.entries.data(), M.entries.size() * sizeof(int),
+                              cudaMemcpyHostToDevice, stream_));
+    PDAL_CUDA(cudaMemcpyAsync((void *)M.d.rows, M.rows.data(), M.rows.size() * sizeof(int), cudaMemcpyHostToDevice,
+                              stream_));
+    k_power_pack<<<std::min((M.ns + 7) / 8, 152 * 8), 256, 0, stream_>>>(M.ns, M.d.entries, M.d.rows, d.rp, d.ci, d.v,
+                                                                         (int *)M.d.ci, (double *)M.d.v);
+    PDAL_CUDA(cudaGetLastError());
+    ++launches_;
+}
+
+/* one of MODE_POWER_*: in slices, or (a long row) in the persistent kernel */
+void FacpSolver::launch_power(int mode, double lam_max) {
+    const bool q = mode != MODE_POWER_A;
+    if ((q ? pow_q_ : pow_a_).ns == 0) {
+        Args a = base_args(mode);
+        a.lam_max = lam_max;
+        launch(a);
+        return;
+    }
+    if (mode == MODE_POWER_QMAX) pack_power(pow_q_, P_.M[MAT_Q]);
+    if (mode == MODE_POWER_A) {
+        pack_power(pow_a_, P_.M[MAT_A]);
+        pack_power(pow_at_, P_.M[MAT_AT]);
+    }
+    PowerArgs a{};
+    a.a = pow_a_.d;
+    a.at = q ? pow_q_.d : pow_at_.d;
+    a.m = q ? H_.n : H_.m;
+    a.n = H_.n;
+    a.v = P_.pv;
+    a.vn = P_.pv2;
+    a.last = P_.out_y;
+    a.dp = P_.pv3;
+    a.part = P_.part;
+    a.bar = P_.bar;
+    a.ctl = P_.ctl;
+    a.bar_extra = P_.bar_extra;
+    a.spin_limit = P_.spin_limit;
+    a.max_iter = p_.sv_max_iter;
+    a.tol = p_.sv_tol;
+    a.tol2 = a.tol > 0.0 ? a.tol * a.tol : 0.0;
+    a.shifted = mode == MODE_POWER_QMIN;
+    a.lam_max = lam_max;
+    const int ns = q ? pow_q_.ns : std::max(pow_a_.ns, pow_at_.ns);
+    const int grid = std::max(1, std::min(sms_, (ns + 1) / 2));
+    PDAL_CUDA(cudaMemsetAsync(P_.bar, 0, sizeof(GridBar), stream_));
+    void *args[] = {(void *)&a};
+    PDAL_CUDA(cudaLaunchCooperativeKernel(q ? (const void *)k_facp_power<true> : (const void *)k_facp_power<false>,
+                                          dim3(grid), dim3(kPowerThreads), args, 0, stream_));
+    ++launches_;
+}
+
 void FacpSolver::power_iterations() {
     const HostQP &H = H_;
     if (qtype_ == Q_SPARSE) { /* solver_state.cu:462-476 */
@@ -589,15 +705,13 @@ void FacpSolver::power_iterations() {
         std::vector<double> v(H.n);
         for (double &x : v) x = (double)rnd.next() / CRandom::kMax;
         PDAL_CUDA(cudaMemcpyAsync(P_.pv, v.data(), H.n * 8, cudaMemcpyHostToDevice, stream_));
-        launch(base_args(MODE_POWER_QMAX));
+        launch_power(MODE_POWER_QMAX, 0.0);
         read_ctl();
         qnorm_ = ctl_.power_value;
         power_iters_q_ += ctl_.power_iters;
         for (double &x : v) x = (double)rnd.next() / CRandom::kMax;
         PDAL_CUDA(cudaMemcpyAsync(P_.pv, v.data(), H.n * 8, cudaMemcpyHostToDevice, stream_));
-        Args a = base_args(MODE_POWER_QMIN);
-        a.lam_max = qnorm_;
-        launch(a);
+        launch_power(MODE_POWER_QMIN, qnorm_);
         read_ctl();
         nonconvexity_ = ctl_.power_value;
         power_iters_q_ += ctl_.power_iters;
@@ -610,7 +724,7 @@ void FacpSolver::power_iterations() {
         std::vector<double> v(H.m);
         for (double &x : v) x = dist(gen);
         PDAL_CUDA(cudaMemcpyAsync(P_.pv, v.data(), H.m * 8, cudaMemcpyHostToDevice, stream_));
-        launch(base_args(MODE_POWER_A));
+        launch_power(MODE_POWER_A, 0.0);
         read_ctl();
         sv_max_ = ctl_.power_value;
         power_iters_a_ = ctl_.power_iters;
