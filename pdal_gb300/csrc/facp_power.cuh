@@ -65,44 +65,56 @@ static __global__ void k_power_pack(int ns, const int2 *__restrict__ entries, co
     }
 }
 
-/* the rows of M times gat, epi(row, sum, red) in the row's lane */
+/* The rows of M times gat, epi(row, sum, red) in the row's lane.  The entries of
+ * the next group, of this slice or the next, are loaded while this group's
+ * gathers are in flight. */
 template <class Epi, class R>
 __device__ __forceinline__ void power_rows(const PowerMat &M, const double *gat, const Epi &epi, R &red) {
     constexpr int U = 4;
     const int lane = threadIdx.x & 31, step = (int)gridDim.x * (kPowerThreads / 32);
     int s = (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x;
-    int2 d, e;
-    if (s < M.ns) {
-        d = __ldg(M.entries + s);
-        e = __ldg(M.rows + (size_t)s * 32 + lane);
-    }
+    if (s >= M.ns) return;
+    int c[U];
+    double w[U];
+    auto entries = [&](const int2 &d, int len, int j, int (&ci)[U], double (&v)[U]) {
+        const size_t at = (size_t)d.x + lane;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (j + u < len) {
+                ci[u] = __ldg(M.ci + at + (j + u) * 32);
+                v[u] = __ldg(M.v + at + (j + u) * 32);
+            }
+    };
+    int2 d = __ldg(M.entries + s), e = __ldg(M.rows + (size_t)s * 32 + lane);
+    entries(d, e.y, 0, c, w);
     while (s < M.ns) {
-        int2 dn, en;
+        int2 dn = make_int2(0, 0), en = make_int2(-1, 0);
         if (s + step < M.ns) {
             dn = __ldg(M.entries + s + step);
             en = __ldg(M.rows + (size_t)(s + step) * 32 + lane);
         }
         typename Epi::In in;
         if (e.x >= 0) in = epi.fetch(e.x);
-        const int *ci = M.ci + d.x + lane;
-        const double *v = M.v + d.x + lane;
         double sum = 0.0;
-        for (int j = 0; j < d.y; j += U) {
-            int c[U];
-            double w[U], g[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u)
-                if (j + u < e.y) {
-                    c[u] = __ldg(ci + (j + u) * 32);
-                    w[u] = __ldg(v + (j + u) * 32);
-                }
+        int j = 0;
+        do {
+            double g[U], wn[U];
+            int cn[U];
 #pragma unroll
             for (int u = 0; u < U; ++u)
                 if (j + u < e.y) g[u] = __ldcg(gat + c[u]);
+            const bool more = j + U < d.y;
+            entries(more ? d : dn, more ? e.y : en.y, more ? j + U : 0, cn, wn);
 #pragma unroll
             for (int u = 0; u < U; ++u)
                 if (j + u < e.y) sum = fma(w[u], g[u], sum);
-        }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                c[u] = cn[u];
+                w[u] = wn[u];
+            }
+            j += U;
+        } while (j < d.y);
         if (e.x >= 0) epi.finish(e.x, sum, in, red);
         s += step;
         d = dn;
