@@ -43,33 +43,46 @@ constexpr int kNoAllocMaxDevices = 64;
 /* The scratch of every call on this device: no call ever allocates. */
 static __device__ __align__(256) double g_partials[kNoAllocMaxBlocks * kNoAllocSlot];
 
-/* Maximum that keeps a NaN: a NaN anywhere in x, A or the bounds must show in
- * max |r| as well as in the norm, or a broken candidate could look feasible. */
-__device__ __forceinline__ double nan_max(double a, double b) { return (a != a || b != b) ? a + b : fmax(a, b); }
+/* |v| as an integer: the bits of non-negative doubles order as the numbers do and
+ * a NaN's above infinity's, so that an integer maximum keeps a NaN -- a NaN
+ * anywhere in x, A or the bounds must show in max |r| as well as in the norm, or
+ * a broken candidate could look feasible -- and leaves the FP64 pipe, which
+ * bounded the reductions, to the sums. */
+using Magnitude = unsigned long long;
+__device__ __forceinline__ Magnitude magnitude(double v) {
+    return (Magnitude)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
 
-/* Deterministic block reduction of (sum, sum, NaN-keeping max); thread 0
- * gets the totals.  sbuf holds 3 * (kThreads / 32) doubles. */
-__device__ __forceinline__ void reduce3(double &s0, double &s1, double &mx, double *sbuf) {
+/* The block's totals in thread 0, the warps' in warp order: `spread` terms are
+ * summed across the lanes first, the others are in lane 0 alone.  sbuf holds
+ * 3 * (kThreads / 32) doubles. */
+__device__ __forceinline__ void reduce3(double &s0, double &s1, Magnitude &mx, bool spread0, bool spread1, double *sbuf) {
     constexpr int NW = kThreads / 32;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (spread0) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-        mx = nan_max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        for (int o = 16; o > 0; o >>= 1) {
+            s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+            mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        }
+    }
+    if (spread1) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s1 += __shfl_xor_sync(0xffffffffu, s1, o);
     }
     if (lane == 0) {
         sbuf[wid] = s0;
         sbuf[NW + wid] = s1;
-        sbuf[2 * NW + wid] = mx;
+        sbuf[2 * NW + wid] = __longlong_as_double((long long)mx);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        s0 = s1 = mx = 0.0;
+        s0 = s1 = 0.0;
+        mx = 0;
         for (int w = 0; w < NW; ++w) {
             s0 += sbuf[w];
             s1 += sbuf[NW + w];
-            mx = nan_max(mx, sbuf[2 * NW + w]);
+            mx = max(mx, magnitude(sbuf[2 * NW + w]));
         }
     }
     __syncthreads();
@@ -85,47 +98,56 @@ __global__ void __launch_bounds__(kThreads) k_primal_kkt_partials(int m, int n, 
                                                                   const double *__restrict__ ub,
                                                                   const double *__restrict__ c,
                                                                   const double *__restrict__ x, double *partials) {
+    asm volatile("griddepcontrol.launch_dependents;");
     __shared__ double sbuf[3 * (kThreads / 32)];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int row = blockIdx.x * kNoAllocRowsPerBlock + warp;
-    double rsq = 0.0, cx = 0.0, rmax = 0.0;
+    double rsq = 0.0, cx = 0.0;
+    Magnitude rmax = 0;
     if (row < m) {
+        const double lo = lb[row], up = ub[row];
         double s = 0.0;
         for (int k = rp[row] + lane; k < rp[row + 1]; k += 32) s = fma(vals[k], x[ci[k]], s);
         s = warp_sum(s);
         if (lane == 0) {
-            const double res = s - fmax(lb[row], fmin(s, ub[row]));
+            const double res = s - fmax(lo, fmin(s, up));
             rsq = res * res;
             /* a NaN row sum gives a NaN residual: fmax/fmin of the projection
              * would turn it into a bound, so carry it explicitly */
-            rmax = (s != s) ? s : fabs(res);
+            rmax = magnitude(s != s ? s : res);
         }
     }
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) cx += c[j] * x[j];
-    reduce3(rsq, cx, rmax, sbuf);
+    reduce3(rsq, cx, rmax, false, (int)blockIdx.x * kThreads < n, sbuf);
     if (threadIdx.x == 0) {
         double *slot = partials + (size_t)blockIdx.x * kNoAllocSlot;
         slot[0] = rsq;
-        slot[1] = rmax;
+        slot[1] = __longlong_as_double((long long)rmax);
         slot[2] = cx;
         slot[3] = 0.0;
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_primal_kkt_finish(int nblocks, const double *__restrict__ partials,
-                                                                double *out) {
+/* One block, resident before the other launch ends (programmatic launch): it
+ * starts with the partials instead of a launch behind them.  A call, with the
+ * integer maxima and the sums of one lane left unshuffled: 2,000 x 5,000 20.6 ->
+ * 11.3 us (10.9 of it on the host), 20,000 x 50,000 78 -> 27 us, 400,000 x 800,000
+ * 1,272 -> 390 us (the FP64 pipe bounded it). */
+__global__ void __launch_bounds__(kThreads) k_primal_kkt_finish(int nblocks, const double *partials, double *out) {
     __shared__ double sbuf[3 * (kThreads / 32)];
-    double rsq = 0.0, cx = 0.0, rmax = 0.0;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    double rsq = 0.0, cx = 0.0;
+    Magnitude rmax = 0;
     for (int b = threadIdx.x; b < nblocks; b += kThreads) {
         const double *slot = partials + (size_t)b * kNoAllocSlot;
         rsq += slot[0];
-        rmax = nan_max(rmax, slot[1]);
+        rmax = max(rmax, magnitude(slot[1]));
         cx += slot[2];
     }
-    reduce3(rsq, cx, rmax, sbuf);
+    reduce3(rsq, cx, rmax, true, true, sbuf);
     if (threadIdx.x == 0) {
         out[0] = sqrt(rsq);
-        out[1] = rmax;
+        out[1] = __longlong_as_double((long long)rmax);
         out[2] = cx;
     }
 }
@@ -218,7 +240,17 @@ int cp_al_gb300_primal_kkt_noalloc(int m, int n, const int *row_ptr, const int *
     const int nblocks = m > 0 ? (m + kNoAllocRowsPerBlock - 1) / kNoAllocRowsPerBlock : 1;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     k_primal_kkt_partials<<<nblocks, kThreads, 0, s>>>(m, n, row_ptr, col_ind, vals, con_lb, con_ub, c, x, scratch);
-    k_primal_kkt_finish<<<1, kThreads, 0, s>>>(nblocks, scratch, out);
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(1);
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, k_primal_kkt_finish, nblocks, (const double *)scratch, out);
+    if (e != cudaSuccess) return fail(std::string("launch: ") + cudaGetErrorString(e));
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail(std::string("launch: ") + cudaGetErrorString(e));
     return 0;
