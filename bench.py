@@ -277,9 +277,8 @@ def run_ours(args, rank, world, local):
     e2e_value = (b_primal + b_dual) * re.iterations * len(rese) * world / dte / 1e9
 
     # time to relative KKT 1e-6 on the plain CP_AL LP (2,000 x 5,000): the
-    # median of three solves of each form after one untimed, with one CUDA
-    # graph per evaluation block (the default) and with the loop on the device
-    # (one cooperative launch per 50 evaluation blocks)
+    # median of three solves of each form after one untimed, as the solver
+    # chooses and with the resident launches in the launches' order of sums
     small = instances.random_lp(2000, 5000, 8, seed=0)
     sp = {"eps": 1e-6, "l_inf_ruiz_iterations": 4}
     kkt = {}
