@@ -48,7 +48,7 @@
  *  1,000,000  FP64     38.2      27.0    22.0
  *             FP32     17.4      25.5    14.6
  * (CpalSolver::flow_form holds the lines drawn from these.)  The tagged power
- * iteration, k_power_flow, takes 6.3 / 7.1 / 11.5 / 16.1 / 23.9 us a step in
+ * iteration, k_power_flow, takes 6.3 / 7.0 / 11.5 / 15.6 / 23.9 us a step in
  * FP64 where five launches took 17.6 / 18.8 / 21.6 / 24.0 / 36.4.
  */
 #pragma once
@@ -213,17 +213,11 @@ constexpr int kSliceUnroll = sizeof(T) == 4 ? 8 : 4;
 template <typename T>
 struct PlainSource {
     const T *p;
-    T scale;
-    bool scaled;
     template <int U>
     __device__ __forceinline__ bool gather(const int (&c)[U], int n, T (&g)[U]) const {
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (u < n) g[u] = __ldcg(p + c[u]);
-        if (scaled) {
-#pragma unroll
-            for (int u = 0; u < U; ++u) g[u] = scale * g[u];
-        }
         return true;
     }
 };
@@ -232,8 +226,6 @@ template <typename T>
 struct TaggedSource {
     TaggedVec<T> v;
     unsigned tag;
-    T scale;
-    bool scaled;
     FlowGuard guard;
     template <int U>
     __device__ __forceinline__ bool gather(const int (&c)[U], int n, T (&g)[U]) const {
@@ -255,10 +247,6 @@ struct TaggedSource {
                 ok = false;
                 break;
             }
-        }
-        if (scaled) {
-#pragma unroll
-            for (int u = 0; u < U; ++u) g[u] = scale * g[u];
         }
         return ok;
     }
@@ -538,14 +526,14 @@ __global__ void __launch_bounds__(kFlowWarps * 32, 1) k_flow(FlowArgs<T> L) {
         if constexpr (BAR) {
             auto wait = [&] { return bar.wait(); };
             auto wait_next = [&] { return i == 1 || bar.wait(); };
-            ok = flow_phase<T>(L.at, sp, PlainSource<T>{L.gat, T(1), false}, ep, tag, L.guard, wait_next) &&
-                 flow_phase<T>(L.a, sd, PlainSource<T>{L.pa.xbar, T(1), false}, ed, tag, L.guard, wait);
+            ok = flow_phase<T>(L.at, sp, PlainSource<T>{L.gat}, ep, tag, L.guard, wait_next) &&
+                 flow_phase<T>(L.a, sd, PlainSource<T>{L.pa.xbar}, ed, tag, L.guard, wait);
         } else {
             if (i == 1)
-                ok = flow_phase<T>(L.at, sp, PlainSource<T>{L.gat, T(1), false}, ep, tag, L.guard, none);
+                ok = flow_phase<T>(L.at, sp, PlainSource<T>{L.gat}, ep, tag, L.guard, none);
             else
-                ok = flow_phase<T>(L.at, sp, TaggedSource<T>{L.ut, tag - 1, T(1), false, L.guard}, ep, tag, L.guard, none);
-            ok = ok && flow_phase<T>(L.a, sd, TaggedSource<T>{L.xt, tag, T(1), false, L.guard}, ed, tag, L.guard, none);
+                ok = flow_phase<T>(L.at, sp, TaggedSource<T>{L.ut, tag - 1, L.guard}, ep, tag, L.guard, none);
+            ok = ok && flow_phase<T>(L.a, sd, TaggedSource<T>{L.xt, tag, L.guard}, ed, tag, L.guard, none);
         }
         if (!ok) {
             if ((threadIdx.x & 31) == 0) atomicExch(&L.st->status, kStatusDeviceError);
@@ -717,8 +705,9 @@ struct FlowStoreEpi {
     struct In {};
     TaggedVec<T> out;
     unsigned tag;
+    T scale; /* the vector's, once per row: FP64 products bound the step */
     __device__ __forceinline__ In fetch(int) const { return In{}; }
-    __device__ __forceinline__ void finish(int j, T s, const In &) const { Tagged<T>::store(out.at(j), s, tag); }
+    __device__ __forceinline__ void finish(int j, T s, const In &) const { Tagged<T>::store(out.at(j), scale * s, tag); }
 };
 
 /* Row i of step k: v_{k+1} = s.  The sums v_k . v_{k+1} and |v_{k+1}|^2, and
@@ -750,7 +739,7 @@ struct FlowPowerEpi {
 
 /*
  * The power iteration of k_power_* in one launch.  Step k = 1, 2, ...:
- * dp = A^T (c_k v_k), v_{k+1} = A dp.  Scaling by c_k = 1/|v_{k-1}| (c_1 =
+ * dp = c_k A^T v_k, v_{k+1} = A dp.  Scaling by c_k = 1/|v_{k-1}| (c_1 =
  * 1/|v_1|) instead of 1/|v_k| keeps the vectors' direction and the Rayleigh
  * quotient
  *   s2_k = v_k . v_{k+1} / (c_k |v_k|^2)
@@ -830,16 +819,16 @@ __global__ void __launch_bounds__(kFlowWarps * 32 + 32, 1) k_power_flow(FlowPowe
             a = s.a;
             b = s.b;
         }
-        FlowStoreEpi<T> ec{L.dt, (unsigned)k};
+        FlowStoreEpi<T> ec{L.dt, (unsigned)k, (T)c};
         bool ok;
         if (k == 1)
-            ok = flow_phase<T>(L.at, sp, PlainSource<T>{L.v0, (T)c, true}, ec, (unsigned)k, L.guard, none);
+            ok = flow_phase<T>(L.at, sp, PlainSource<T>{L.v0}, ec, (unsigned)k, L.guard, none);
         else
-            ok = flow_phase<T>(L.at, sp, TaggedSource<T>{L.vt, (unsigned)(k - 1), (T)c, true, L.guard}, ec, (unsigned)k,
+            ok = flow_phase<T>(L.at, sp, TaggedSource<T>{L.vt, (unsigned)(k - 1), L.guard}, ec, (unsigned)k,
                                L.guard, none);
         double s[4] = {0.0, 0.0, 0.0, 0.0};
         FlowPowerEpi<T> er{L, (unsigned)k, a, b, s};
-        ok = ok && flow_phase<T>(L.a, sd, TaggedSource<T>{L.dt, (unsigned)k, T(1), false, L.guard}, er, (unsigned)k,
+        ok = ok && flow_phase<T>(L.a, sd, TaggedSource<T>{L.dt, (unsigned)k, L.guard}, er, (unsigned)k,
                                  L.guard, none);
         if (!ok) return;
         if (warp < active) flow_publish(f, active, (unsigned)k, s, L.sums + (size_t)(k & 3) * gridDim.x * 4);
