@@ -57,7 +57,7 @@ def build_ref() -> list[Path]:
     functions and an empty PSLP_stats.h).  Their internal headers include the
     CUDA headers for declarations only; nothing of CUDA is linked.  Returns
     the built objects, or [] where the reference sources are absent."""
-    if not REFERENCE.exists():
+    if not (REFERENCE / "LP/CP_AL/src/mps_parser.c").exists():  # no checkout, or an empty directory
         return []
     REF_OUT.mkdir(exist_ok=True)
     out = []
