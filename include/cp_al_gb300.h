@@ -186,6 +186,10 @@ typedef struct {
                                      the captured graphs).  1 and -1 (default) = yes (an iteration of
                                      the large LP: FP32 98.9 -> 97 us, FP64 183 -> 178 us), 0 = one
                                      after the other.  Results are bit-identical either way */
+    int resident_fail_launch;     /* fault injection for tests: this resident launch of the solver (1 = the
+                                     first, in the order they are issued or captured) gives up at the
+                                     first wait that is not over at once; the solve then fails with a
+                                     message.  0 (default) = none: a wait gives up after about 2 s */
 } cp_al_gb300_options_t;
 
 /* Statistics of the last solve on this thread (for benchmarks and tests). */

@@ -946,6 +946,7 @@ void oracle_cpal_default_options(cp_al_gb300_options_t *o) {
     o->dynamic_eval_ratio = 1e4;
     o->dynamic_eval_bootstrap_iters = 0;
     o->dual_concurrent = -1;
+    o->resident_fail_launch = 0;
 }
 
 /* LP/CP_AL/src/utils.cu:361-394 (reflection coefficient without the

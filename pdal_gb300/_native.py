@@ -223,6 +223,7 @@ class CpalOptions(C.Structure):
         ("dynamic_eval_ratio", C.c_double),
         ("dynamic_eval_bootstrap_iters", C.c_int),
         ("dual_concurrent", C.c_int),
+        ("resident_fail_launch", C.c_int),
     ]
 
 

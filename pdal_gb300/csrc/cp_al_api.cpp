@@ -394,6 +394,7 @@ void cp_al_gb300_default_options(cp_al_gb300_options_t *o) {
     o->dynamic_eval_ratio = 1e4;
     o->dynamic_eval_bootstrap_iters = 0;
     o->dual_concurrent = -1;
+    o->resident_fail_launch = 0;
 }
 
 /* Each variable is read the way the reference reads it

@@ -337,7 +337,8 @@ class CpalSolver {
     template <typename... K, typename... A>
     void launch_coop(void (*kern)(K...), int threads, size_t smem, A... args);
     /* polls of an L2 round trip each: a wait gives up after about 2 s */
-    FlowGuard guard() const { return FlowGuard{dev_err_, 1 << 22}; }
+    FlowGuard next_guard() { return FlowGuard{dev_err_, ++resident_launches_ == O_.resident_fail_launch ? 0 : 1 << 22}; }
+    int resident_launches_ = 0;
     bool staged_rows() const { return O_.primal_staged == 2; }
     void check_device_error();
     int *At_ci_hot_ = nullptr;
@@ -1219,7 +1220,7 @@ FlowPowerArgs<T> CpalSolver::power_args() {
     L.vt = tagged_u<T>();
     L.sums = flow_sums_;
     L.ps = ps_;
-    L.guard = guard();
+    L.guard = next_guard();
     return L;
 }
 
@@ -1760,7 +1761,7 @@ void CpalSolver::launch_flow(int F) {
     L.st = st_;
     L.wt = weights<T>(wt_, wtf_);
     L.F = F;
-    L.guard = guard();
+    L.guard = next_guard();
     L.bar = flow_bar_;
     const size_t smem = flow_smem_[sizeof(T) == 8];
     if (flow_form<T>() == Flow::barrier) {

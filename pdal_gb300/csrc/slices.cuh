@@ -127,20 +127,25 @@ struct FlowGuard {
 
 /* Grid barrier of the worker warps (for the problems whose gathers are too
  * many to poll): one release-add per CTA on a counter that is zero at launch,
- * then an acquire poll until all CTAs of this barrier have arrived. */
+ * then an acquire poll until all CTAs of this barrier have arrived.  All worker
+ * warps of a CTA call every wait(), a warp whose own work gave up (!good) with
+ * them: a warp that left by itself would leave its CTA's others in bar.sync for
+ * good.  The same wait() then returns false in all of them, without polling. */
 struct FlowBarrier {
     unsigned *count;
-    int *ok; /* shared */
+    int *ok;     /* shared */
+    int *failed; /* shared, zero at first */
     FlowGuard guard;
     unsigned target;
     __device__ __forceinline__ void workers() const { asm volatile("bar.sync 1, %0;" ::"n"(kFlowWarps * 32) : "memory"); }
-    __device__ __forceinline__ bool wait() {
+    __device__ __forceinline__ bool wait(bool good_so_far) {
         target += gridDim.x;
+        if (!good_so_far) *(volatile int *)failed = 1;
         workers();
         if (threadIdx.x == 0) {
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
-            int spins = 0, good = 1;
-            for (;;) {
+            int spins = 0, good = *(volatile int *)failed == 0;
+            while (good) {
                 unsigned v;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
                 if (v >= target) break;
@@ -508,38 +513,47 @@ struct FlowDualEpi {
 template <typename T, bool BETA, bool BAR>
 __global__ void __launch_bounds__(kFlowWarps * 32, 1) k_flow(FlowArgs<T> L) {
     extern __shared__ __align__(16) unsigned char flow_smem[];
-    __shared__ int bar_ok;
-    if (L.st->status) return; /* set between launches only */
+    __shared__ int bar_ok, bar_failed;
+    /* one read for the CTA: a CTA that gives up sets the status while others
+     * start, and a CTA of which a part left would not get through its barriers */
+    if (__syncthreads_or(threadIdx.x == 0 ? L.st->status : 0)) return;
+    if (threadIdx.x == 0) bar_failed = 0;
     unsigned char *at = flow_smem;
     const SliceShare<T> sp = slice_share(L.at, at), sd = slice_share(L.a, at);
     Coefs<T> k;
     load_coefs(L.st, k);
     __syncthreads();
-    FlowBarrier bar{L.bar, &bar_ok, L.guard, 0u};
+    FlowBarrier bar{L.bar, &bar_ok, &bar_failed, L.guard, 0u};
     auto none = [] { return true; };
+    bool good = true; /* no wait of this warp has given up */
     for (int i = 1; i <= L.F; ++i) {
         const T w = L.wt[i].w, omw = L.wt[i].omw;
         const unsigned tag = (unsigned)i;
         FlowPrimalEpi<T, BAR> ep{L, k, w, omw, tag};
         FlowDualEpi<T, BETA, BAR> ed{L, k, w, omw, tag};
-        bool ok;
         if constexpr (BAR) {
-            auto wait = [&] { return bar.wait(); };
-            auto wait_next = [&] { return i == 1 || bar.wait(); };
-            ok = flow_phase<T>(L.at, sp, PlainSource<T>{L.gat}, ep, tag, L.guard, wait_next) &&
-                 flow_phase<T>(L.a, sd, PlainSource<T>{L.pa.xbar}, ed, tag, L.guard, wait);
+            /* a phase is false where its barrier failed, in every warp of the
+             * CTA, or where this warp gave up on a long row's parts: then the
+             * next barrier takes the CTA out */
+            bool left = false;
+            auto wait = [&] {
+                left = !bar.wait(good);
+                return !left;
+            };
+            auto wait_next = [&] { return i == 1 || wait(); };
+            good = flow_phase<T>(L.at, sp, PlainSource<T>{L.gat}, ep, tag, L.guard, wait_next);
+            if (!left) good = flow_phase<T>(L.a, sd, PlainSource<T>{L.pa.xbar}, ed, tag, L.guard, wait);
+            if (left) break;
         } else {
             if (i == 1)
-                ok = flow_phase<T>(L.at, sp, PlainSource<T>{L.gat}, ep, tag, L.guard, none);
+                good = flow_phase<T>(L.at, sp, PlainSource<T>{L.gat}, ep, tag, L.guard, none);
             else
-                ok = flow_phase<T>(L.at, sp, TaggedSource<T>{L.ut, tag - 1, L.guard}, ep, tag, L.guard, none);
-            ok = ok && flow_phase<T>(L.a, sd, TaggedSource<T>{L.xt, tag, L.guard}, ed, tag, L.guard, none);
-        }
-        if (!ok) {
-            if ((threadIdx.x & 31) == 0) atomicExch(&L.st->status, kStatusDeviceError);
-            return;
+                good = flow_phase<T>(L.at, sp, TaggedSource<T>{L.ut, tag - 1, L.guard}, ep, tag, L.guard, none);
+            good = good && flow_phase<T>(L.a, sd, TaggedSource<T>{L.xt, tag, L.guard}, ed, tag, L.guard, none);
+            if (!good) break;
         }
     }
+    if (!good && (threadIdx.x & 31) == 0) atomicExch(&L.st->status, kStatusDeviceError);
 }
 
 /* ------------------------------------------------------------------ */
