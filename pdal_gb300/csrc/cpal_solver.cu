@@ -1052,7 +1052,6 @@ void CpalSolver::upload() {
     arena_.reserve_measured();
     alloc_all();
     upload_alloc_sec = now_sec() - t_alloc;
-    PDAL_CUDA(cudaMemsetAsync(dev_err_, 0, sizeof(int), stream_));
     for (int q = 0; q < 2; ++q)
         if (!eq_long_h_[q].empty())
             PDAL_CUDA(cudaMemcpyAsync(eq_long_[q], eq_long_h_[q].data(), eq_long_h_[q].size() * sizeof(int),
@@ -1440,6 +1439,8 @@ void CpalSolver::setup_device() {
     fp32_iters = 0;
     fp32_phase_ = O_.precision == CP_AL_GB300_FP32_REFINE;
     const size_t n = n_, m = m_, nnz = nnz_;
+    /* a solve of this session whose waits ran out does not stop this one */
+    PDAL_CUDA(cudaMemsetAsync(dev_err_, 0, sizeof(int), stream_));
     auto d2d = [&](void *dst, const void *src, size_t b) {
         if (b) PDAL_CUDA(cudaMemcpyAsync(dst, src, b, cudaMemcpyDeviceToDevice, stream_));
     };

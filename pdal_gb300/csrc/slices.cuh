@@ -115,9 +115,10 @@ struct TaggedVec {
 struct FlowGuard {
     int *err;
     int limit;
-    __device__ __forceinline__ bool expired(int &spins) const {
+    /* `weight`: polls of this wait in the time of an L2 round trip */
+    __device__ __forceinline__ bool expired(int &spins, int weight = 1) const {
         ++spins;
-        if (spins > limit) {
+        if (spins > limit * weight) {
             atomicExch(err, 2);
             return true;
         }
@@ -691,8 +692,10 @@ __device__ __forceinline__ void flow_ready(FlowSums &f, unsigned rec) {
 __device__ __forceinline__ bool flow_wait(FlowSums &f, unsigned rec, const FlowGuard &guard) {
     int spins = 0;
     bool ok = true;
+    /* of shared memory, tens of cycles a poll: as long as the service warp may
+     * wait for the other CTAs, whose verdict this one would otherwise preempt */
     while (f.ready[rec & 3] != (int)rec)
-        if (guard.expired(spins)) {
+        if (guard.expired(spins, 32)) {
             ok = false;
             break;
         }

@@ -37,3 +37,30 @@ def test_barrier_form_with_long_rows_gives_up(lp_lib, m, n, k, precision):
     with pytest.raises(RuntimeError, match=MESSAGE):
         lp.solve(d, p, fail)
     assert lp.solve(d, p, o).iterations == 200
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(2000, 5000), (9000, 21000)], ids=["tagged", "barrier"])
+@pytest.mark.parametrize("launch", [1, 2], ids=["power", "iterations"])
+def test_waits_run_out_and_a_new_solve_succeeds(lp_lib, shape, launch):
+    """FP64: the power iteration's launch (the service warp and the warps that
+    wait for it in shared memory) and the iterations' launch in both forms."""
+    d = I.random_lp(*shape, 8, seed=4)
+    p = {"eps": 1e-14, "iteration_limit": 200, "sv_max_iter": 50}
+    with pytest.raises(RuntimeError, match=MESSAGE):
+        lp.solve(d, p, {"resident_fail_launch": launch})
+    assert lp.solve(d, p, {}).iterations == 200
+
+
+@pytest.mark.gpu
+def test_a_session_solves_again_after_a_wait_ran_out(lp_lib):
+    """The error of one solve is not the next one's."""
+    d = I.random_lp(2000, 5000, 8, seed=4)
+    p = {"eps": 1e-14, "iteration_limit": 200, "sv_max_iter": 50}
+    s = lp.LPSession(d, p, {"resident_fail_launch": 1})
+    with pytest.raises(RuntimeError, match=MESSAGE):
+        s.solve()
+    again = s.solve()
+    s.close()
+    assert again.iterations == 200
+    assert again.stats["lambda_est"] == lp.solve(d, p, {}).stats["lambda_est"]
