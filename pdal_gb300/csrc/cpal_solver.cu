@@ -330,8 +330,7 @@ class CpalSolver {
     }
     template <typename T>
     SliceDev<T> slice_dev(int which) const;
-    template <typename T>
-    FlowPowerArgs<T> power_args();
+    FlowPowerArgs power_args();
     template <typename T>
     void launch_flow(int F);
     template <typename... K, typename... A>
@@ -1210,13 +1209,16 @@ static void launch_pdl(void (*kern)(KArgs...), int grid, cudaStream_t stream, Ar
     PDAL_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
 }
 
-template <typename T>
-FlowPowerArgs<T> CpalSolver::power_args() {
-    FlowPowerArgs<T> L{};
-    L.at = slice_dev<T>(0);
-    L.a = slice_dev<T>(1);
-    L.dt = tagged_x<T>();
-    L.vt = tagged_u<T>();
+FlowPowerArgs CpalSolver::power_args() {
+    FlowPowerArgs L{};
+    L.at = slice_dev<double>(0);
+    L.a = slice_dev<double>(1);
+    L.v0 = tmp_m_;
+    /* m-sized buffers the iteration has not started to use */
+    double *hist[4] = {tmp_m2_, tmp_m_, v64_.y, v64_.yh};
+    for (int q = 0; q < 4; ++q) L.hist[q] = hist[q];
+    L.dt = tagged_x<double>();
+    L.vt = tagged_u<double>();
     L.sums = flow_sums_;
     L.ps = ps_;
     L.guard = next_guard();
@@ -1247,7 +1249,7 @@ void CpalSolver::power_iteration() {
     /* plain form: FP64 over the evaluation plans; chosen form: FP32 over the
      * iteration plans and the FP32 matrix copies (made before this call) */
     const bool f32 = fp32_phase_;
-    const bool flow = h.max_iter > 0 && O_.persistent_loop != 1 && flow_smem_[f32 ? 0 : 1] > 0;
+    const bool flow = !f32 && h.max_iter > 0 && O_.persistent_loop != 1 && flow_smem_[1] > 0;
     std::vector<double> v0;
     if (!f32 && !flow) {
         /* the plain form of a large LP keeps the host's logarithm and order of
@@ -1275,20 +1277,9 @@ void CpalSolver::power_iteration() {
     PDAL_LAUNCH_CHECK();
     launches += 1;
     if (flow) {
-        /* m-sized buffers the iteration has not started to use */
         clear_flow();
-        const int steps = std::min(h.max_iter, INT32_MAX - 8);
-        auto run = [&](auto args, auto kern, size_t smem) {
-            using T = std::remove_pointer_t<decltype(args.v0)>;
-            args.v0 = (T *)tmp_m_;
-            T *hist[4] = {(T *)tmp_m2_, (T *)tmp_m_, (T *)v64_.y, (T *)v64_.yh};
-            for (int q = 0; q < 4; ++q) args.hist[q] = hist[q];
-            launch_coop(kern, (kFlowWarps + 1) * 32, smem, args, steps);
-        };
-        if (f32)
-            run(power_args<float>(), k_power_flow<float>, flow_smem_[0]);
-        else
-            run(power_args<double>(), k_power_flow<double>, flow_smem_[1]);
+        launch_coop(k_power_flow, (kFlowWarps + 1) * 32, flow_smem_[1], power_args(),
+                    std::min(h.max_iter, INT32_MAX - 8));
         launches += 1;
         PDAL_CUDA(cudaMemcpyAsync(h_ps_, ps_, sizeof(PowerState), cudaMemcpyDeviceToHost, stream_));
         d2h += sizeof(PowerState);

@@ -706,49 +706,47 @@ __device__ __forceinline__ bool flow_wait(FlowSums &f, unsigned rec, const FlowG
 /* ------------------------------------------------------------------ */
 /* sigma_max(A)^2                                                      */
 /* ------------------------------------------------------------------ */
-template <typename T>
 struct FlowPowerArgs {
-    SliceDev<T> at, a;
-    T *v0;              /* the start vector, plain */
-    T *hist[4];         /* the last vectors, each read by the thread that wrote it */
-    TaggedVec<T> dt, vt; /* A^T v and v, tags zero before the launch */
+    SliceDev<double> at, a;
+    double *v0;         /* the start vector, plain */
+    double *hist[4];    /* the last vectors, each read by the thread that wrote it */
+    TaggedVec<double> dt, vt; /* A^T v and v, tags zero before the launch */
     Tagged<double>::Word *sums; /* [CTAs' sums, totals][record & 3][CTA][4], tags zero before the launch */
     PowerState *ps;
     FlowGuard guard;
 };
 
-template <typename T>
 struct FlowStoreEpi {
     struct In {};
-    TaggedVec<T> out;
+    TaggedVec<double> out;
     unsigned tag;
-    T scale; /* the vector's, once per row: FP64 products bound the step */
+    double scale; /* the vector's, once per row: FP64 products bound the step */
     __device__ __forceinline__ In fetch(int) const { return In{}; }
-    __device__ __forceinline__ void finish(int j, T s, const In &) const { Tagged<T>::store(out.at(j), scale * s, tag); }
+    __device__ __forceinline__ void finish(int j, double s, const In &) const {
+        Tagged<double>::store(out.at(j), scale * s, tag);
+    }
 };
 
 /* Row i of step k: v_{k+1} = s.  The sums v_k . v_{k+1} and |v_{k+1}|^2, and
  * step k-2's share |v_{k-1} a - v_{k-2} b|^2 of the residual. */
-template <typename T>
 struct FlowPowerEpi {
     struct In {
-        T v, v1, v2;
+        double v, v1, v2;
     };
-    const FlowPowerArgs<T> &L;
+    const FlowPowerArgs &L;
     unsigned k;
     double a, b;
     double *s;
     __device__ __forceinline__ In fetch(int i) const {
-        return In{L.hist[k & 3][i], k > 2 ? L.hist[(k - 1) & 3][i] : T(0), k > 2 ? L.hist[(k - 2) & 3][i] : T(0)};
+        return In{L.hist[k & 3][i], k > 2 ? L.hist[(k - 1) & 3][i] : 0.0, k > 2 ? L.hist[(k - 2) & 3][i] : 0.0};
     }
-    __device__ __forceinline__ void finish(int i, T x, const In &in) const {
-        Tagged<T>::store(L.vt.at(i), x, k);
+    __device__ __forceinline__ void finish(int i, double x, const In &in) const {
+        Tagged<double>::store(L.vt.at(i), x, k);
         L.hist[(k + 1) & 3][i] = x;
-        const double w = (double)x;
-        s[0] += (double)in.v * w;
-        s[1] += w * w;
+        s[0] += in.v * x;
+        s[1] += x * x;
         if (k > 2) {
-            const double d = (double)in.v1 * a - b * (double)in.v2;
+            const double d = in.v1 * a - b * in.v2;
             s[2] += d * d;
         }
     }
@@ -756,24 +754,26 @@ struct FlowPowerEpi {
 
 /*
  * The power iteration of k_power_* in one launch.  Step k = 1, 2, ...:
- * dp = c_k A^T v_k, v_{k+1} = A dp.  Scaling by c_k = 1/|v_{k-1}| (c_1 =
- * 1/|v_1|) instead of 1/|v_k| keeps the vectors' direction and the Rayleigh
- * quotient
- *   s2_k = v_k . v_{k+1} / (c_k |v_k|^2)
- * (the norms stay bounded: ln|v_{k+1}| = ln s2 + ln|v_k| - ln|v_{k-1}|), and
- * takes the grid's sums off the critical path: those of step k are used from
- * step k+2 on.  The residual of step k, |v_{k+1} / (c_k |v_k|) - s2_k v_k / |v_k||,
+ * dp = c_k A^T v_k, v_{k+1} = A dp.  Any c_k keeps the vectors' direction and
+ * the Rayleigh quotient
+ *   s2_k = v_k . v_{k+1} / (c_k |v_k|^2),
+ * so 1/|v_k| is foretold from the sums of step k-2, which takes the grid's sums
+ * off the critical path: with the growth g = |v_{k-1}| / (c_{k-2} |v_{k-2}|) of
+ * that step, |v_k| is about c_{k-1} g |v_{k-1}|.  Then |v_{k+1}| = g_k g_{k-1} /
+ * g_{k-2}, about the largest eigenvalue, as with 1/|v_k| itself (c_1 and c_2
+ * are that, c_3 = c_2; 1/|v_{k-1}| for c_k, one scalar less, swings the norm up
+ * to the eigenvalue's square, whose own square leaves the range of a double for
+ * entries of 1e39).  The residual of step k, |v_{k+1} / (c_k |v_k|) - s2_k v_k / |v_k||,
  * is added element by element in step k+2 and tested in step k+4; the steps
  * run in excess change nothing, s2 is that of the step whose residual passed.
  * One warp more than the workers (the service warp) collects the sums.
  */
 struct FlowScalars {
-    double c, a, b; /* scale of step rec + 2; the residual's coefficients of step rec */
+    double c, a, b; /* scale of step rec + 2 (rec = 1: of step 2 too); the residual's coefficients of step rec */
     int done;
 };
 
-template <typename T>
-__global__ void __launch_bounds__(kFlowWarps * 32 + 32, 1) k_power_flow(FlowPowerArgs<T> L, int max_steps) {
+static __global__ void __launch_bounds__(kFlowWarps * 32 + 32, 1) k_power_flow(FlowPowerArgs L, int max_steps) {
     extern __shared__ __align__(16) unsigned char flow_smem[];
     __shared__ FlowSums f;
     __shared__ FlowScalars sc[4];
@@ -783,18 +783,16 @@ __global__ void __launch_bounds__(kFlowWarps * 32 + 32, 1) k_power_flow(FlowPowe
         f.ready[threadIdx.x] = 0;
     }
     unsigned char *at = flow_smem;
-    const SliceShare<T> sp = slice_share(L.at, at), sd = slice_share(L.a, at);
+    const SliceShare<double> sp = slice_share(L.at, at), sd = slice_share(L.a, at);
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const double c1 = L.ps->inv, n1 = L.ps->vsq, tol = L.ps->tol;
-    const double c2 = 1.0 / sqrt(n1);
     const int active = max(1, min(sd.s1 - sd.s0, kFlowWarps)); /* warps that publish sums */
     /* every step whose residual may be wanted, plus the four that follow it */
     const int last = max_steps + 4;
     if (warp == kFlowWarps) {
         double ck[4], nk[4], s2k[4]; /* by step & 3 */
         ck[1] = c1;
-        ck[2] = c2;
         nk[1] = n1;
         for (int rec = 1; rec <= last; ++rec) {
             double tot;
@@ -803,7 +801,8 @@ __global__ void __launch_bounds__(kFlowWarps * 32 + 32, 1) k_power_flow(FlowPowe
                          rr = __shfl_sync(0xffffffffu, tot, 2);
             const double c = ck[rec & 3], n = nk[rec & 3];
             nk[(rec + 1) & 3] = nn;
-            ck[(rec + 2) & 3] = 1.0 / sqrt(nn);
+            if (rec == 1) ck[2] = 1.0 / sqrt(nn);
+            ck[(rec + 2) & 3] = c * sqrt(n) / (ck[(rec + 1) & 3] * nn);
             const double s2 = dot / (c * n), inv_n = 1.0 / sqrt(n);
             /* the residual of step rec - 2 */
             const int step = rec - 2;
@@ -827,25 +826,26 @@ __global__ void __launch_bounds__(kFlowWarps * 32 + 32, 1) k_power_flow(FlowPowe
     if (flow_idle(L.at, sp, active)) return;
     auto none = [] { return true; };
     for (int k = 1; k <= last; ++k) {
-        double c = k == 1 ? c1 : c2, a = 0.0, b = 0.0;
-        if (k > 2) {
-            if (!flow_wait(f, (unsigned)(k - 2), L.guard)) return;
-            const FlowScalars s = sc[(k - 2) & 3];
+        double c = c1, a = 0.0, b = 0.0;
+        if (k > 1) {
+            const int rec = max(k - 2, 1); /* c_3 = c_2 */
+            if (!flow_wait(f, (unsigned)rec, L.guard)) return;
+            const FlowScalars s = sc[rec & 3];
             if (s.done) return;
             c = s.c;
             a = s.a;
             b = s.b;
         }
-        FlowStoreEpi<T> ec{L.dt, (unsigned)k, (T)c};
+        FlowStoreEpi ec{L.dt, (unsigned)k, c};
         bool ok;
         if (k == 1)
-            ok = flow_phase<T>(L.at, sp, PlainSource<T>{L.v0}, ec, (unsigned)k, L.guard, none);
+            ok = flow_phase<double>(L.at, sp, PlainSource<double>{L.v0}, ec, (unsigned)k, L.guard, none);
         else
-            ok = flow_phase<T>(L.at, sp, TaggedSource<T>{L.vt, (unsigned)(k - 1), L.guard}, ec, (unsigned)k,
+            ok = flow_phase<double>(L.at, sp, TaggedSource<double>{L.vt, (unsigned)(k - 1), L.guard}, ec, (unsigned)k,
                                L.guard, none);
         double s[4] = {0.0, 0.0, 0.0, 0.0};
-        FlowPowerEpi<T> er{L, (unsigned)k, a, b, s};
-        ok = ok && flow_phase<T>(L.a, sd, TaggedSource<T>{L.dt, (unsigned)k, L.guard}, er, (unsigned)k,
+        FlowPowerEpi er{L, (unsigned)k, a, b, s};
+        ok = ok && flow_phase<double>(L.a, sd, TaggedSource<double>{L.dt, (unsigned)k, L.guard}, er, (unsigned)k,
                                  L.guard, none);
         if (!ok) return;
         if (warp < active) flow_publish(f, active, (unsigned)k, s, L.sums + (size_t)(k & 3) * gridDim.x * 4);
