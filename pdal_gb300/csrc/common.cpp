@@ -182,13 +182,18 @@ HostPlan plan_rows(int nr, const int *rp, int S) {
     return P;
 }
 
-HostSlices plan_slices(const HostPlan &P, const int *rp, int lanes) {
+HostSlices plan_slices(const HostPlan &P, const int *rp, int lanes, int chain) {
     HostSlices Q;
     /* lanes per row of a STREAM block, as rowblock_run_at chooses them */
     auto group = [&](int nrows) {
         if (lanes > 0) return lanes;
         int g = 32;
         while (g > 1 && g * nrows > kThreads) g >>= 1;
+        return g;
+    };
+    /* of a row of `len` entries, no lane with more than `chain` of them */
+    auto widen = [&](int g, int len) {
+        while (chain > 0 && g < 32 && len > (long long)g * chain) g *= 2;
         return g;
     };
     /* the blocks, STREAM blocks merged into windows where the lanes are given */
@@ -205,8 +210,13 @@ HostSlices plan_slices(const HostPlan &P, const int *rp, int lanes) {
     const int nw = (int)win.size();
     std::vector<int> first((size_t)nw + 1, 0);
     for (int b = 0; b < nw; ++b) {
-        const int nrows = win[b].second - win[b].first;
-        first[b + 1] = first[b] + (win[b].second < 0 ? 8 : (nrows * group(nrows) + 31) / 32);
+        first[b + 1] = first[b] + 8;
+        if (win[b].second < 0) continue;
+        const int nrows = win[b].second - win[b].first, g0 = group(nrows);
+        int with[33] = {0}; /* rows by their lanes */
+        for (int r = win[b].first; r < win[b].second; ++r) with[widen(g0, rp[r + 1] - rp[r])]++;
+        first[b + 1] = first[b];
+        for (int g = g0; g <= 32; g *= 2) first[b + 1] += (with[g] * g + 31) / 32;
     }
     Q.n = first[nw];
     Q.desc.resize(4 * (size_t)Q.n);
@@ -232,7 +242,7 @@ HostSlices plan_slices(const HostPlan &P, const int *rp, int lanes) {
                 }
                 continue;
             }
-            const int nrows = win[b].second - win[b].first, g = group(nrows), per = 32 / g;
+            const int nrows = win[b].second - win[b].first, g0 = group(nrows);
             int longest = 0;
             for (int r = win[b].first; r < win[b].second; ++r) longest = std::max(longest, rp[r + 1] - rp[r]);
             at.assign((size_t)longest + 2, 0);
@@ -241,16 +251,20 @@ HostSlices plan_slices(const HostPlan &P, const int *rp, int lanes) {
             rows.resize(nrows);
             for (int r = win[b].first; r < win[b].second; ++r)
                 rows[at[longest - (rp[r + 1] - rp[r])]++] = {rp[r] - rp[r + 1], r};
-            for (int q = 0; q < nrows; q += per) {
-                const size_t s = (size_t)first[b] + q / per;
+            size_t s = (size_t)first[b];
+            for (int q = 0; q < nrows; ++s) {
+                const int g = widen(g0, -rows[q].first);
+                int end = q; /* the slice's rows: as long as they have the same lanes */
+                while (end < nrows && end < q + 32 / g && widen(g0, -rows[end].first) == g) ++end;
                 Q.desc[4 * s + 1] = (-rows[q].first + g - 1) / g;
                 Q.desc[4 * s + 2] = g;
                 Q.desc[4 * s + 3] = 0;
                 for (int l = 0; l < 32; ++l) {
-                    const bool in = q + l / g < nrows;
+                    const bool in = q + l / g < end;
                     Q.rl[64 * s + 2 * l] = in ? rows[q + l / g].second : -1;
                     Q.rl[64 * s + 2 * l + 1] = in ? std::max(-rows[q + l / g].first - l % g + g - 1, 0) / g : 0;
                 }
+                q = end;
             }
         }
     });

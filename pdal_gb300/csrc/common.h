@@ -126,8 +126,9 @@ struct HostSlices {
 };
 /* `lanes` = 0: a row's lanes are those of rowblock_run_at (bit-identical
  * sums); > 0: that many lanes (a power of two) for every row that is not
- * long, over windows of 1,024 rows sorted by length. */
-HostSlices plan_slices(const HostPlan &P, const int *rp, int lanes);
+ * long, over windows of 1,024 rows sorted by length; with `chain` > 0 a row gets
+ * twice the lanes, up to 32, until none holds more than `chain` entries. */
+HostSlices plan_slices(const HostPlan &P, const int *rp, int lanes, int chain = 0);
 /* First slice of each of `parts` contiguous ranges of about equal cost
  * (parts + 1 entries), and the largest number of packed entries in one. */
 std::vector<int> split_slices(const HostSlices &Q, int parts, long long &most);

@@ -338,6 +338,7 @@ class CpalSolver {
     /* polls of an L2 round trip each: a wait gives up after about 2 s */
     FlowGuard next_guard() { return FlowGuard{dev_err_, ++resident_launches_ == O_.resident_fail_launch ? 0 : 1 << 22}; }
     int resident_launches_ = 0;
+    bool has_long() const { return A_.it.hp.nlong > 0 || At_.it.hp.nlong > 0; }
     bool staged_rows() const { return O_.primal_staged == 2; }
     void check_device_error();
     int *At_ci_hot_ = nullptr;
@@ -815,12 +816,18 @@ void CpalSolver::plan_flow() {
         for (int q = 0; q < 2; ++q) {
             Sliced &l = sl_[f][q];
             const int nr = q ? m_ : n_;
-            /* as few lanes per row as give every SM a slice */
-            int lanes = 0;
-            if (O_.persistent_loop != 1)
+            /* as few lanes per row as give every SM a slice, and more for the
+             * rows that are longer than most: a lane's entries are dependent
+             * rounds of gathers that every CTA waits for (20,000 x 50,000 with
+             * five rows of 370 entries among rows of 20, FP64: 67 us an
+             * iteration with them in one lane each, 15.4 so, 19.7 by launches) */
+            int lanes = 0, chain = 0;
+            if (O_.persistent_loop != 1) {
                 for (lanes = 1; lanes < 32 && (long long)nr * lanes < 32LL * sms && 2LL * lanes * nr <= nnz_;) lanes *= 2;
+                chain = std::max(8, 2 * (int)(nnz_ / ((long long)nr * lanes) + 1));
+            }
             l.h = plan_slices((q ? A_ : At_).it.hp, q ? prob_->constraint_matrix_row_pointers : At_host_.rp.data(),
-                              lanes);
+                              lanes, chain);
             long long most = 0;
             l.cut = split_slices(l.h, sms, most);
             bytes += (size_t)most * entry;
@@ -1278,7 +1285,7 @@ void CpalSolver::power_iteration() {
     launches += 1;
     if (flow) {
         clear_flow();
-        launch_coop(k_power_flow, (kFlowWarps + 1) * 32, flow_smem_[1], power_args(),
+        launch_coop(has_long() ? k_power_flow<true> : k_power_flow<false>, (kFlowWarps + 1) * 32, flow_smem_[1], power_args(),
                     std::min(h.max_iter, INT32_MAX - 8));
         launches += 1;
         PDAL_CUDA(cudaMemcpyAsync(h_ps_, ps_, sizeof(PowerState), cudaMemcpyDeviceToHost, stream_));
@@ -1758,9 +1765,13 @@ void CpalSolver::launch_flow(int F) {
     const size_t smem = flow_smem_[sizeof(T) == 8];
     if (flow_form<T>() == Flow::barrier) {
         PDAL_CUDA(cudaMemsetAsync(flow_bar_, 0, sizeof(unsigned), stream_));
-        launch_coop(beta_on_ ? k_flow<T, true, true> : k_flow<T, false, true>, kFlowWarps * 32, smem, L);
+        launch_coop(has_long() ? (beta_on_ ? k_flow<T, true, true, true> : k_flow<T, false, true, true>)
+                               : (beta_on_ ? k_flow<T, true, true, false> : k_flow<T, false, true, false>),
+                    kFlowWarps * 32, smem, L);
     } else {
-        launch_coop(beta_on_ ? k_flow<T, true, false> : k_flow<T, false, false>, kFlowWarps * 32, smem, L);
+        launch_coop(has_long() ? (beta_on_ ? k_flow<T, true, false, true> : k_flow<T, false, false, true>)
+                               : (beta_on_ ? k_flow<T, true, false, false> : k_flow<T, false, false, false>),
+                    kFlowWarps * 32, smem, L);
     }
 }
 

@@ -9,7 +9,8 @@
  * warp's loads of column indices and values are whole 128-byte lines and no
  * staging, row pointers or block barriers stand between a load and its
  * product.  Rows are sorted by length within a window, so the lanes of a
- * slice end together; each has the fewest lanes that give every SM a slice.
+ * slice end together; each has the fewest lanes that give every SM a slice, and
+ * more where it is long, since a lane's entries are dependent rounds of gathers.
  * Few lanes matter most in FP64: an FP64 instruction holds an SM's FP64 pipe
  * for 19 cycles however many lanes are active, and a dependent one waits 64
  * (measured), so with the row-block engine's 16 lanes a row the epilogues, in
@@ -337,16 +338,63 @@ __device__ __forceinline__ SliceShare<T> slice_share(const SliceDev<T> &M, unsig
     return r;
 }
 
+/* The sum of long row `li` of `len` entries from its parts, as they are
+ * published under `tag`: eight per piece in order, then the pieces in FP64 in
+ * order.  Not inlined: its registers would spill into the products' loops. */
+template <typename T>
+__device__ __noinline__ bool flow_long_sum(const typename Tagged<T>::Word *part, int4 li, int len, int S, unsigned tag,
+                                           FlowGuard guard, T &sum) {
+    const int lane = threadIdx.x & 31;
+    double tot = 0.0;
+    bool ok = true;
+    for (int q0 = 0; q0 < li.y; q0 += 32) {
+        T t = T(0);
+        if (q0 + lane < li.y) {
+            /* the piece's parts polled together: one after the other they take
+             * a round trip to L2 each */
+            const int parts = min(8, (min(S, len - (q0 + lane) * S) + 31) / 32);
+            const typename Tagged<T>::Word *p = part + (size_t)(li.z + q0 + lane) * 8;
+            T v[8];
+            unsigned need = (1u << parts) - 1u;
+            int spins = 0;
+            while (need) {
+                typename Tagged<T>::Word w[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (need & (1u << u)) w[u] = Tagged<T>::load(p + u);
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if ((need & (1u << u)) && Tagged<T>::is(w[u], tag)) {
+                        v[u] = Tagged<T>::value(w[u]);
+                        need &= ~(1u << u);
+                    }
+                if (need && guard.expired(spins)) {
+                    ok = false;
+                    break;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (u < parts) t += v[u];
+        }
+        const int n = min(32, li.y - q0);
+        for (int k = 0; k < n; ++k) tot += (double)__shfl_sync(0xffffffffu, t, k);
+    }
+    sum = (T)tot;
+    return !__any_sync(0xffffffffu, !ok);
+}
+
 /* One product over the slices of this warp: every row's sum goes to
  * epi.finish(row, sum, epi.fetch(row)), whose inputs are loaded before the
  * gathers wait.  The parts of a long row publish their sums under `tag`; the
- * warp that holds the row's first part collects them after its own slices --
- * eight per piece in order, then the pieces in FP64 in order, as
- * rowblock_run_at adds them.  A part without entries publishes nothing (it
- * waits for nothing and could run ahead).  wait() returns when a plain source
- * is complete (a tagged one waits by itself).  Returns false for the whole
- * warp when a wait gave up. */
-template <typename T, class Src, class Epi, class Wait>
+ * warp that holds the row's first part collects them after its own slices, in
+ * the order of rowblock_run_at.  A part without entries publishes nothing (it
+ * waits for nothing and could run ahead).  Without LONG there are no long rows:
+ * their code costs the products' loops registers (20,000 x 50,000 in FP64 with
+ * it 16.5 us an iteration and 17.4 a power step, without 14.9 and 14.5).  wait()
+ * returns when a plain source is complete (a tagged one waits by itself).
+ * Returns false for the whole warp when a wait gave up. */
+template <bool LONG, typename T, class Src, class Epi, class Wait>
 __device__ __forceinline__ bool flow_phase(const SliceDev<T> &M, const SliceShare<T> &sh, const Src &src, Epi &epi,
                                            unsigned tag, const FlowGuard &guard, Wait wait) {
     const int lane = threadIdx.x & 31, first = sh.s0 + (int)(threadIdx.x >> 5);
@@ -370,46 +418,25 @@ __device__ __forceinline__ bool flow_phase(const SliceDev<T> &M, const SliceShar
         if (d.z > 0) {
             for (int o = d.z >> 1; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, d.z);
             if (lead) epi.finish(e.x, acc, in);
-        } else if (d.y > 0) {
+        } else if (LONG && d.y > 0) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
             if (lane == 0) Tagged<T>::store(M.part + d.w, acc, tag);
         }
     }
-    if (M.nlong == 0) return true;
-    for (int s = first; s < sh.s1; s += kFlowWarps) {
-        const int4 d = M.desc[s];
-        if (d.z > 0) continue;
-        const int4 li = M.linfo[M.rl[(size_t)s * 32].x]; /* {row, pieces, first piece, first entry} */
-        if (d.w != 8 * li.z) continue;
-        typename Epi::In in;
-        if (lane == 0) in = epi.fetch(li.x);
-        const int len = M.rp[li.x + 1] - li.w;
-        double tot = 0.0;
-        bool ok = true;
-        for (int q0 = 0; q0 < li.y; q0 += 32) {
-            T t = T(0);
-            if (q0 + lane < li.y) {
-                const int parts = min(8, (min(M.S, len - (q0 + lane) * M.S) + 31) / 32);
-                for (int w = 0; w < parts && ok; ++w) {
-                    const typename Tagged<T>::Word *p = M.part + (size_t)(li.z + q0 + lane) * 8 + w;
-                    typename Tagged<T>::Word x = Tagged<T>::load(p);
-                    int spins = 0;
-                    while (!Tagged<T>::is(x, tag)) {
-                        if (guard.expired(spins)) {
-                            ok = false;
-                            break;
-                        }
-                        x = Tagged<T>::load(p);
-                    }
-                    t += Tagged<T>::value(x);
-                }
-            }
-            const int n = min(32, li.y - q0);
-            for (int k = 0; k < n; ++k) tot += (double)__shfl_sync(0xffffffffu, t, k);
+    if constexpr (LONG) {
+        if (M.nlong == 0) return true;
+        for (int s = first; s < sh.s1; s += kFlowWarps) {
+            const int4 d = M.desc[s];
+            if (d.z > 0) continue;
+            const int4 li = M.linfo[M.rl[(size_t)s * 32].x]; /* {row, pieces, first piece, first entry} */
+            if (d.w != 8 * li.z) continue;
+            typename Epi::In in;
+            if (lane == 0) in = epi.fetch(li.x);
+            T tot;
+            if (!flow_long_sum<T>(M.part, li, M.rp[li.x + 1] - li.w, M.S, tag, guard, tot)) return false;
+            if (lane == 0) epi.finish(li.x, tot, in);
         }
-        if (__any_sync(0xffffffffu, !ok)) return false;
-        if (lane == 0) epi.finish(li.x, (T)tot, in);
     }
     return true;
 }
@@ -511,7 +538,7 @@ struct FlowDualEpi {
     }
 };
 
-template <typename T, bool BETA, bool BAR>
+template <typename T, bool BETA, bool BAR, bool LONG>
 __global__ void __launch_bounds__(kFlowWarps * 32, 1) k_flow(FlowArgs<T> L) {
     extern __shared__ __align__(16) unsigned char flow_smem[];
     __shared__ int bar_ok, bar_failed;
@@ -542,15 +569,15 @@ __global__ void __launch_bounds__(kFlowWarps * 32, 1) k_flow(FlowArgs<T> L) {
                 return !left;
             };
             auto wait_next = [&] { return i == 1 || wait(); };
-            good = flow_phase<T>(L.at, sp, PlainSource<T>{L.gat}, ep, tag, L.guard, wait_next);
-            if (!left) good = flow_phase<T>(L.a, sd, PlainSource<T>{L.pa.xbar}, ed, tag, L.guard, wait);
+            good = flow_phase<LONG, T>(L.at, sp, PlainSource<T>{L.gat}, ep, tag, L.guard, wait_next);
+            if (!left) good = flow_phase<LONG, T>(L.a, sd, PlainSource<T>{L.pa.xbar}, ed, tag, L.guard, wait);
             if (left) break;
         } else {
             if (i == 1)
-                good = flow_phase<T>(L.at, sp, PlainSource<T>{L.gat}, ep, tag, L.guard, none);
+                good = flow_phase<LONG, T>(L.at, sp, PlainSource<T>{L.gat}, ep, tag, L.guard, none);
             else
-                good = flow_phase<T>(L.at, sp, TaggedSource<T>{L.ut, tag - 1, L.guard}, ep, tag, L.guard, none);
-            good = good && flow_phase<T>(L.a, sd, TaggedSource<T>{L.xt, tag, L.guard}, ed, tag, L.guard, none);
+                good = flow_phase<LONG, T>(L.at, sp, TaggedSource<T>{L.ut, tag - 1, L.guard}, ep, tag, L.guard, none);
+            good = good && flow_phase<LONG, T>(L.a, sd, TaggedSource<T>{L.xt, tag, L.guard}, ed, tag, L.guard, none);
             if (!good) break;
         }
     }
@@ -773,7 +800,8 @@ struct FlowScalars {
     int done;
 };
 
-static __global__ void __launch_bounds__(kFlowWarps * 32 + 32, 1) k_power_flow(FlowPowerArgs L, int max_steps) {
+template <bool LONG>
+__global__ void __launch_bounds__(kFlowWarps * 32 + 32, 1) k_power_flow(FlowPowerArgs L, int max_steps) {
     extern __shared__ __align__(16) unsigned char flow_smem[];
     __shared__ FlowSums f;
     __shared__ FlowScalars sc[4];
@@ -839,13 +867,13 @@ static __global__ void __launch_bounds__(kFlowWarps * 32 + 32, 1) k_power_flow(F
         FlowStoreEpi ec{L.dt, (unsigned)k, c};
         bool ok;
         if (k == 1)
-            ok = flow_phase<double>(L.at, sp, PlainSource<double>{L.v0}, ec, (unsigned)k, L.guard, none);
+            ok = flow_phase<LONG, double>(L.at, sp, PlainSource<double>{L.v0}, ec, (unsigned)k, L.guard, none);
         else
-            ok = flow_phase<double>(L.at, sp, TaggedSource<double>{L.vt, (unsigned)(k - 1), L.guard}, ec, (unsigned)k,
+            ok = flow_phase<LONG, double>(L.at, sp, TaggedSource<double>{L.vt, (unsigned)(k - 1), L.guard}, ec, (unsigned)k,
                                L.guard, none);
         double s[4] = {0.0, 0.0, 0.0, 0.0};
         FlowPowerEpi er{L, (unsigned)k, a, b, s};
-        ok = ok && flow_phase<double>(L.a, sd, TaggedSource<double>{L.dt, (unsigned)k, L.guard}, er, (unsigned)k,
+        ok = ok && flow_phase<LONG, double>(L.a, sd, TaggedSource<double>{L.dt, (unsigned)k, L.guard}, er, (unsigned)k,
                                  L.guard, none);
         if (!ok) return;
         if (warp < active) flow_publish(f, active, (unsigned)k, s, L.sums + (size_t)(k & 3) * gridDim.x * 4);
