@@ -208,13 +208,22 @@ HostSlices plan_slices(const HostPlan &P, const int *rp, int lanes, int chain) {
             win.emplace_back(d[0], d[1]);
     }
     const int nw = (int)win.size();
-    std::vector<int> first((size_t)nw + 1, 0);
+    std::vector<int> first((size_t)nw + 1, 0), shortest(nw, 0), longest(nw, 0);
     for (int b = 0; b < nw; ++b) {
         first[b + 1] = first[b] + 8;
         if (win[b].second < 0) continue;
         const int nrows = win[b].second - win[b].first, g0 = group(nrows);
+        int &lo = shortest[b], &hi = longest[b];
+        lo = INT32_MAX;
+        for (int r = win[b].first; r < win[b].second; ++r) {
+            lo = std::min(lo, rp[r + 1] - rp[r]);
+            hi = std::max(hi, rp[r + 1] - rp[r]);
+        }
         int with[33] = {0}; /* rows by their lanes */
-        for (int r = win[b].first; r < win[b].second; ++r) with[widen(g0, rp[r + 1] - rp[r])]++;
+        if (widen(g0, lo) == widen(g0, hi))
+            with[widen(g0, lo)] = nrows;
+        else
+            for (int r = win[b].first; r < win[b].second; ++r) with[widen(g0, rp[r + 1] - rp[r])]++;
         first[b + 1] = first[b];
         for (int g = g0; g <= 32; g *= 2) first[b + 1] += (with[g] * g + 31) / 32;
     }
@@ -243,27 +252,31 @@ HostSlices plan_slices(const HostPlan &P, const int *rp, int lanes, int chain) {
                 continue;
             }
             const int nrows = win[b].second - win[b].first, g0 = group(nrows);
-            int longest = 0;
-            for (int r = win[b].first; r < win[b].second; ++r) longest = std::max(longest, rp[r + 1] - rp[r]);
-            at.assign((size_t)longest + 2, 0);
-            for (int r = win[b].first; r < win[b].second; ++r) at[longest - (rp[r + 1] - rp[r]) + 1]++;
-            for (int q = 0; q <= longest; ++q) at[q + 1] += at[q];
             rows.resize(nrows);
-            for (int r = win[b].first; r < win[b].second; ++r)
-                rows[at[longest - (rp[r + 1] - rp[r])]++] = {rp[r] - rp[r + 1], r};
+            if (shortest[b] == longest[b]) {
+                for (int r = win[b].first; r < win[b].second; ++r) rows[r - win[b].first] = {-longest[b], r};
+            } else {
+                const int hi = longest[b];
+                at.assign((size_t)hi + 2, 0);
+                for (int r = win[b].first; r < win[b].second; ++r) at[hi - (rp[r + 1] - rp[r]) + 1]++;
+                for (int q = 0; q <= hi; ++q) at[q + 1] += at[q];
+                for (int r = win[b].first; r < win[b].second; ++r)
+                    rows[at[hi - (rp[r + 1] - rp[r])]++] = {rp[r] - rp[r + 1], r};
+            }
             size_t s = (size_t)first[b];
             for (int q = 0; q < nrows; ++s) {
-                const int g = widen(g0, -rows[q].first);
+                const int g = widen(g0, -rows[q].first), lg = __builtin_ctz((unsigned)g);
                 int end = q; /* the slice's rows: as long as they have the same lanes */
-                while (end < nrows && end < q + 32 / g && widen(g0, -rows[end].first) == g) ++end;
-                Q.desc[4 * s + 1] = (-rows[q].first + g - 1) / g;
+                while (end < nrows && end < q + (32 >> lg) && widen(g0, -rows[end].first) == g) ++end;
+                Q.desc[4 * s + 1] = (-rows[q].first + g - 1) >> lg;
                 Q.desc[4 * s + 2] = g;
                 Q.desc[4 * s + 3] = 0;
-                for (int l = 0; l < 32; ++l) {
-                    const bool in = q + l / g < end;
-                    Q.rl[64 * s + 2 * l] = in ? rows[q + l / g].second : -1;
-                    Q.rl[64 * s + 2 * l + 1] = in ? std::max(-rows[q + l / g].first - l % g + g - 1, 0) / g : 0;
-                }
+                int *rl = &Q.rl[64 * s];
+                for (int r = q; r < q + (32 >> lg); ++r)
+                    for (int l = 0; l < g; ++l, rl += 2) {
+                        rl[0] = r < end ? rows[r].second : -1;
+                        rl[1] = r < end ? std::max(-rows[r].first - l + g - 1, 0) >> lg : 0;
+                    }
                 q = end;
             }
         }

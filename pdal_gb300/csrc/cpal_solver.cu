@@ -286,18 +286,20 @@ class CpalSolver {
     std::vector<int> eq_long_h_[2];
     int *eq_long_[2] = {nullptr, nullptr}; /* [A, A^T] */
     void setup_staged();
-    /* LPs that fit on the chip: sliced copies of A^T and A (index 0, 1) in each
-     * precision (FP32, FP64), the iterations of an evaluation block and the
-     * sigma_max estimate as resident launches (slices.cuh) */
+    /* LPs that fit on the chip: sliced copies of A^T and A (index 0, 1), one
+     * plan with values in each precision (FP32, FP64) that fits, the iterations
+     * of an evaluation block and the sigma_max estimate as resident launches
+     * (slices.cuh) */
     struct Sliced {
         HostSlices h;
         std::vector<int> cut;
         int4 *desc = nullptr;
         int2 *rl = nullptr;
         int *ci = nullptr, *cta = nullptr;
-        void *val = nullptr;
-        ulonglong2 *part = nullptr;
-    } sl_[2][2];
+        float *v32 = nullptr;
+        double *v64 = nullptr;
+        ulonglong2 *part = nullptr; /* of the precision that iterates */
+    } sl_[2];
     int flow_grid_ = 0;             /* CTAs of the resident launches */
     int flow_shift_[2] = {0, 0};    /* spacing of the tagged x-bar and u */
     template <typename T>
@@ -809,88 +811,90 @@ void CpalSolver::plan_flow() {
      * SMs while many poll it cost several exchanges' time (40,000 + 400 entries,
      * exchange alone: 26,900 cycles packed, 6,600 with 128 bytes per entry) */
     for (int q = 0; q < 2; ++q) flow_shift_[q] = (q ? m_ : n_) <= 1024 ? 4 : (q ? m_ : n_) <= 4096 ? 2 : 0;
-    for (int f = fp32_phase_ ? 0 : 1; f < 2; ++f) {
-        const size_t entry = sizeof(int) + (f ? sizeof(double) : sizeof(float));
-        if ((size_t)nnz_ * 2 * entry > sms * kFlowSmem) continue;
-        size_t bytes = 0;
-        for (int q = 0; q < 2; ++q) {
-            Sliced &l = sl_[f][q];
-            const int nr = q ? m_ : n_;
-            /* as few lanes per row as give every SM a slice, and more for the
-             * rows that are longer than most: a lane's entries are dependent
-             * rounds of gathers that every CTA waits for (20,000 x 50,000 with
-             * five rows of 370 entries among rows of 20, FP64: 67 us an
-             * iteration with them in one lane each, 15.4 so, 19.7 by launches) */
-            int lanes = 0, chain = 0;
-            if (O_.persistent_loop != 1) {
-                for (lanes = 1; lanes < 32 && (long long)nr * lanes < 32LL * sms && 2LL * lanes * nr <= nnz_;) lanes *= 2;
-                chain = std::max(8, 2 * (int)(nnz_ / ((long long)nr * lanes) + 1));
-            }
-            l.h = plan_slices((q ? A_ : At_).it.hp, q ? prob_->constraint_matrix_row_pointers : At_host_.rp.data(),
-                              lanes, chain);
-            long long most = 0;
-            l.cut = split_slices(l.h, sms, most);
-            bytes += (size_t)most * entry;
+    auto bytes = [](int f, size_t entries) { return entries * (sizeof(int) + (f ? 8 : 4)); };
+    const int first = fp32_phase_ ? 0 : 1;
+    if (bytes(first, 2 * (size_t)nnz_) > sms * kFlowSmem) return;
+    size_t entries = 0; /* of a CTA */
+    for (int q = 0; q < 2; ++q) {
+        Sliced &l = sl_[q];
+        const int nr = q ? m_ : n_;
+        /* as few lanes per row as give every SM a slice, and more for the
+         * rows that are longer than most: a lane's entries are dependent
+         * rounds of gathers that every CTA waits for (20,000 x 50,000 with
+         * five rows of 370 entries among rows of 20, FP64: 67 us an
+         * iteration with them in one lane each, 15.4 so, 19.7 by launches) */
+        int lanes = 0, chain = 0;
+        if (O_.persistent_loop != 1) {
+            for (lanes = 1; lanes < 32 && (long long)nr * lanes < 32LL * sms && 2LL * lanes * nr <= nnz_;) lanes *= 2;
+            chain = std::max(8, 2 * (int)(nnz_ / ((long long)nr * lanes) + 1));
         }
-        if (bytes <= kFlowSmem) flow_smem_[f] = std::max<size_t>(bytes, 16);
+        l.h = plan_slices((q ? A_ : At_).it.hp, q ? prob_->constraint_matrix_row_pointers : At_host_.rp.data(), lanes,
+                          chain);
+        long long most = 0;
+        l.cut = split_slices(l.h, sms, most);
+        entries += (size_t)most;
     }
+    for (int f = first; f < 2; ++f)
+        if (bytes(f, entries) <= kFlowSmem) flow_smem_[f] = std::max<size_t>(bytes(f, entries), 16);
+    if (!flow_smem_[0] && !flow_smem_[1])
+        for (Sliced &l : sl_) l.h = HostSlices();
 }
 
 void CpalSolver::alloc_flow() {
-    for (int f = 0; f < 2; ++f)
-        for (int q = 0; q < 2 && flow_smem_[f]; ++q) {
-            Sliced &l = sl_[f][q];
-            const size_t len = (size_t)std::max(l.h.len, 1LL);
-            l.desc = arena_.take<int4>(std::max(l.h.n, 1));
-            l.rl = arena_.take<int2>(32 * (size_t)std::max(l.h.n, 1));
-            l.cta = arena_.take<int>((size_t)flow_grid_ + 1);
-            l.ci = arena_.take<int>(len);
-            l.val = f ? (void *)arena_.take<double>(len) : (void *)arena_.take<float>(len);
-            l.part = arena_.take<ulonglong2>(8 * (size_t)std::max((q ? A_ : At_).it.hp.npieces, 1));
-        }
-    if (flow_smem_[0] || flow_smem_[1]) {
-        flow_xt_ = arena_.take<ulonglong2>((size_t)n_ << flow_shift_[0]);
-        flow_ut_ = arena_.take<ulonglong2>((size_t)m_ << flow_shift_[1]);
-        flow_bar_ = arena_.take<unsigned>(1);
-        flow_sums_ = arena_.take<ulonglong2>(32 * (size_t)flow_grid_);
+    if (!flow_smem_[0] && !flow_smem_[1]) return;
+    for (int q = 0; q < 2; ++q) {
+        Sliced &l = sl_[q];
+        const size_t len = (size_t)std::max(l.h.len, 1LL);
+        l.desc = arena_.take<int4>(std::max(l.h.n, 1));
+        l.rl = arena_.take<int2>(32 * (size_t)std::max(l.h.n, 1));
+        l.cta = arena_.take<int>((size_t)flow_grid_ + 1);
+        l.ci = arena_.take<int>(len);
+        if (flow_smem_[0]) l.v32 = arena_.take<float>(len);
+        if (flow_smem_[1]) l.v64 = arena_.take<double>(len);
+        l.part = arena_.take<ulonglong2>(8 * (size_t)std::max((q ? A_ : At_).it.hp.npieces, 1));
     }
+    flow_xt_ = arena_.take<ulonglong2>((size_t)n_ << flow_shift_[0]);
+    flow_ut_ = arena_.take<ulonglong2>((size_t)m_ << flow_shift_[1]);
+    flow_bar_ = arena_.take<unsigned>(1);
+    flow_sums_ = arena_.take<ulonglong2>(32 * (size_t)flow_grid_);
 }
 
 void CpalSolver::upload_flow() {
+    if (!flow_xt_) return;
     auto up = [&](void *dst, const std::vector<int> &v) {
         if (v.empty()) return;
         PDAL_CUDA(cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice, stream_));
         h2d += (int64_t)(v.size() * sizeof(int));
     };
-    for (int f = 0; f < 2; ++f)
-        for (int q = 0; q < 2 && flow_smem_[f]; ++q) {
-            Sliced &l = sl_[f][q];
-            const DevMatrix &M = q ? A_ : At_;
-            up(l.desc, l.h.desc);
-            up(l.rl, l.h.rl);
-            up(l.cta, l.cut);
-            k_slice_pack<<<grid_for(32LL * l.h.n), kThreads, 0, stream_>>>(l.h.n, l.desc, l.rl, M.it.d.linfo, S_it_,
-                                                                          M.rp, (const int *)M.ci, l.ci);
-            PDAL_LAUNCH_CHECK();
-        }
+    for (int q = 0; q < 2; ++q) {
+        Sliced &l = sl_[q];
+        const DevMatrix &M = q ? A_ : At_;
+        up(l.desc, l.h.desc);
+        up(l.rl, l.h.rl);
+        up(l.cta, l.cut);
+        k_slice_pack<<<grid_for(32LL * l.h.n), kThreads, 0, stream_>>>(l.h.n, l.desc, l.rl, M.it.d.linfo, S_it_, M.rp,
+                                                                      (const int *)M.ci, l.ci);
+        PDAL_LAUNCH_CHECK();
+    }
 }
 
 /* the equilibrated values in slices, in each precision the solve runs in */
 void CpalSolver::pack_flow() {
-    for (int f = 0; f < 2; ++f)
-        for (int q = 0; q < 2 && flow_smem_[f]; ++q) {
-            const Sliced &l = sl_[f][q];
-            const DevMatrix &M = q ? A_ : At_;
-            const int g = grid_for(32LL * l.h.n);
-            if (f)
-                k_slice_pack<<<g, kThreads, 0, stream_>>>(l.h.n, l.desc, l.rl, M.it.d.linfo, S_it_, M.rp,
-                                                          (const double *)M.v, (double *)l.val);
-            else
-                k_slice_pack<<<g, kThreads, 0, stream_>>>(l.h.n, l.desc, l.rl, M.it.d.linfo, S_it_, M.rp,
-                                                          (const double *)M.v, (float *)l.val);
+    if (!flow_xt_) return;
+    for (int q = 0; q < 2; ++q) {
+        const Sliced &l = sl_[q];
+        const DevMatrix &M = q ? A_ : At_;
+        const int g = grid_for(32LL * l.h.n);
+        auto pack = [&](auto *to) {
+            if (!to) return;
+            k_slice_pack<<<g, kThreads, 0, stream_>>>(l.h.n, l.desc, l.rl, M.it.d.linfo, S_it_, M.rp,
+                                                      (const double *)M.v, to);
             PDAL_LAUNCH_CHECK();
             launches += 1;
-        }
+        };
+        pack(l.v32);
+        pack(l.v64);
+    }
 }
 
 /* no entry carries a tag (before an estimate, and before the iteration) */
@@ -899,20 +903,18 @@ void CpalSolver::clear_flow() {
     PDAL_CUDA(cudaMemsetAsync(flow_xt_, 0, sizeof(ulonglong2) * ((size_t)n_ << flow_shift_[0]), stream_));
     PDAL_CUDA(cudaMemsetAsync(flow_ut_, 0, sizeof(ulonglong2) * ((size_t)m_ << flow_shift_[1]), stream_));
     PDAL_CUDA(cudaMemsetAsync(flow_sums_, 0, sizeof(ulonglong2) * 32 * (size_t)flow_grid_, stream_));
-    for (int f = 0; f < 2; ++f)
-        for (int q = 0; q < 2 && flow_smem_[f]; ++q)
-            PDAL_CUDA(cudaMemsetAsync(sl_[f][q].part, 0,
-                                      sizeof(ulonglong2) * 8 * (size_t)std::max((q ? A_ : At_).it.hp.npieces, 1),
-                                      stream_));
+    for (int q = 0; q < 2; ++q)
+        PDAL_CUDA(cudaMemsetAsync(sl_[q].part, 0,
+                                  sizeof(ulonglong2) * 8 * (size_t)std::max((q ? A_ : At_).it.hp.npieces, 1), stream_));
 }
 
 template <typename T>
 SliceDev<T> CpalSolver::slice_dev(int q) const {
-    const Sliced &l = sl_[sizeof(T) == 8][q];
+    const Sliced &l = sl_[q];
     const DevMatrix &M = q ? A_ : At_;
-    return SliceDev<T>{l.desc, l.rl, l.ci, (const T *)l.val, l.cta, M.it.d.linfo, M.rp,
-                       (typename Tagged<T>::Word *)l.part, l.h.n, M.it.d.nlong, S_it_,
-                       O_.persistent_loop == 1};
+    const void *val = sizeof(T) == 8 ? (const void *)l.v64 : (const void *)l.v32;
+    return SliceDev<T>{l.desc, l.rl, l.ci, (const T *)val, l.cta, M.it.d.linfo, M.rp,
+                       (typename Tagged<T>::Word *)l.part, l.h.n, M.it.d.nlong, S_it_, O_.persistent_loop == 1};
 }
 
 /* a cooperative launch of one CTA per SM (also inside a stream capture) */
@@ -1170,11 +1172,10 @@ void CpalSolver::upload() {
         PDAL_CUDA(cudaMemsetAsync(y00_, 0, std::max<size_t>(m, 1) * sizeof(double), stream_));
     PDAL_CUDA(cudaStreamSynchronize(stream_));
     At_host_ = HostCsr(); /* host transpose no longer needed */
-    for (auto &f : sl_)
-        for (auto &l : f) {
-            l.h.desc = std::vector<int>();
-            l.h.rl = std::vector<int>();
-        }
+    for (Sliced &l : sl_) {
+        l.h.desc = std::vector<int>();
+        l.h.rl = std::vector<int>();
+    }
     pan_host_.pmap = decltype(pan_host_.pmap)();
     pan_host_.off = decltype(pan_host_.off)();
     upload_sec = now_sec() - t_up;
