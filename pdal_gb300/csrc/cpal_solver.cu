@@ -148,6 +148,17 @@ struct IterVecs {
 
 } // namespace
 
+/* Resident launches need the packed matrices of both products in the shared
+ * memory of one CTA per SM, in the precision that iterates. */
+constexpr size_t kFlowSmem = 224 * 1024;
+/* Rows of up to this many entries sit in the lanes of one warp, also where the
+ * row blocks of a small LP are shorter: a longer one costs its eight warps an
+ * exchange per piece. */
+constexpr int kFlowLongRow = 1024;
+/* slices a CTA of 16 warps has on average at most where rows get more lanes:
+ * CTAs of equal cost differ in their slices */
+constexpr int kFlowSlices = 12;
+
 class CpalSolver {
   public:
     CpalSolver(const lp_problem_t *prob, const cp_al_parameters_t *params, const cp_al_gb300_options_t *opts)
@@ -292,8 +303,9 @@ class CpalSolver {
      * (slices.cuh) */
     struct Sliced {
         HostSlices h;
-        std::vector<int> cut;
-        int4 *desc = nullptr;
+        std::vector<int> cut, linfo_h;
+        int S = 0, nlong = 0, npieces = 0; /* rows of more than S entries, in pieces */
+        int4 *desc = nullptr, *linfo = nullptr;
         int2 *rl = nullptr;
         int *ci = nullptr, *cta = nullptr;
         float *v32 = nullptr;
@@ -320,15 +332,30 @@ class CpalSolver {
     void clear_flow();
     enum class Flow { launches, tagged, barrier };
     /* How the iteration's products run.  The lines lie where the measured
-     * times cross (the table in slices.cuh): polling pays up to about 90,000
-     * nonzeros in both precisions; above, FP64 gains from the resident form
-     * at every size that fits, FP32, whose launches take half the time, from
-     * about 600,000 on.  `timing` brackets single launches. */
+     * times cross (the table in slices.cuh; `rows`: rows and columns, whose
+     * epilogues bound every form where there are few nonzeros to each).
+     * FP64: polling pays up to 200,000 nonzeros, the barrier form above; LPs of
+     * fewer nonzeros than rows gain up to 150,000 and nothing beyond, those of
+     * more than 250,000 rows nothing before the launches' row blocks grow.
+     * FP32, whose launches take half the time: polling up to 100,000 nonzeros
+     * where there are 1.5 or more to a row, up to 30,000 otherwise, where the
+     * barrier form gains to 150,000; and the barrier form from 630,000 on where
+     * a lane per row fills the warps (fewer rows have chains that the launches
+     * cut shorter).  `timing` brackets single launches. */
     template <typename T>
     Flow flow_form() const {
         if (flow_smem_[sizeof(T) == 8] == 0 || O_.timing != 0) return Flow::launches;
-        if (nnz_ <= 90000 || O_.persistent_loop == 1) return Flow::tagged;
-        return sizeof(T) == 8 || nnz_ >= 600000 ? Flow::barrier : Flow::launches;
+        if (O_.persistent_loop == 1) return Flow::tagged;
+        const long long rows = (long long)m_ + n_;
+        if (sizeof(T) == 8) {
+            if (nnz_ > 150000 && (rows > nnz_ || (rows > 250000 && nnz_ <= 600000))) return Flow::launches;
+            return nnz_ <= 200000 ? Flow::tagged : Flow::barrier;
+        }
+        if (nnz_ <= 30000) return Flow::tagged;
+        if (2LL * nnz_ < 3 * rows && nnz_ <= 150000) return Flow::barrier;
+        if (nnz_ <= 100000) return Flow::tagged;
+        const bool filled = 2LL * std::min(m_, n_) > 32LL * kFlowSlices * flow_grid_;
+        return nnz_ >= 630000 && 5LL * nnz_ >= 7 * rows && filled ? Flow::barrier : Flow::launches;
     }
     template <typename T>
     SliceDev<T> slice_dev(int which) const;
@@ -340,7 +367,7 @@ class CpalSolver {
     /* polls of an L2 round trip each: a wait gives up after about 2 s */
     FlowGuard next_guard() { return FlowGuard{dev_err_, ++resident_launches_ == O_.resident_fail_launch ? 0 : 1 << 22}; }
     int resident_launches_ = 0;
-    bool has_long() const { return A_.it.hp.nlong > 0 || At_.it.hp.nlong > 0; }
+    bool has_long() const { return sl_[0].nlong > 0 || sl_[1].nlong > 0; }
     bool staged_rows() const { return O_.primal_staged == 2; }
     void check_device_error();
     int *At_ci_hot_ = nullptr;
@@ -793,10 +820,6 @@ void CpalSolver::setup_staged() {
     });
 }
 
-/* Resident launches need the packed matrices of both products in the shared
- * memory of one CTA per SM, in the precision that iterates. */
-constexpr size_t kFlowSmem = 224 * 1024;
-
 void CpalSolver::plan_flow() {
     flow_grid_ = 0;
     flow_smem_[0] = flow_smem_[1] = 0;
@@ -818,18 +841,28 @@ void CpalSolver::plan_flow() {
     for (int q = 0; q < 2; ++q) {
         Sliced &l = sl_[q];
         const int nr = q ? m_ : n_;
-        /* as few lanes per row as give every SM a slice, and more for the
-         * rows that are longer than most: a lane's entries are dependent
-         * rounds of gathers that every CTA waits for (20,000 x 50,000 with
-         * five rows of 370 entries among rows of 20, FP64: 67 us an
-         * iteration with them in one lane each, 15.4 so, 19.7 by launches) */
+        /* Lanes per row: doubled until every SM has a slice, and on to four
+         * entries a lane while the slices still have a warp each (a lane's
+         * entries are dependent rounds of gathers; two slices of half the
+         * length in one warp take longer than one, for the epilogues).  Then
+         * more for the rows that are longer than most: every CTA waits for the
+         * longest lane. */
         int lanes = 0, chain = 0;
         if (O_.persistent_loop != 1) {
-            for (lanes = 1; lanes < 32 && (long long)nr * lanes < 32LL * sms && 2LL * lanes * nr <= nnz_;) lanes *= 2;
-            chain = std::max(8, 2 * (int)(nnz_ / ((long long)nr * lanes) + 1));
+            const long long rows = nr, one_warp = 32LL * kFlowSlices * sms;
+            for (lanes = 1; lanes < 32 && 2 * lanes * rows <= nnz_; lanes *= 2)
+                if (rows * lanes >= 32LL * sms && (4 * lanes * rows >= nnz_ || 2 * lanes * rows > one_warp)) break;
+            chain = std::max(8, (int)((2LL * nnz_ + rows * lanes - 1) / (rows * lanes)));
         }
-        l.h = plan_slices((q ? A_ : At_).it.hp, q ? prob_->constraint_matrix_row_pointers : At_host_.rp.data(), lanes,
-                          chain);
+        const int *rp = q ? prob_->constraint_matrix_row_pointers : At_host_.rp.data();
+        const HostPlan &it = (q ? A_ : At_).it.hp;
+        const HostPlan own = O_.persistent_loop == 1 || S_it_ >= kFlowLongRow ? HostPlan() : plan_rows(nr, rp, kFlowLongRow);
+        const HostPlan &plan = own.nblocks > 0 ? own : it;
+        l.S = plan.S;
+        l.nlong = plan.nlong;
+        l.npieces = plan.npieces;
+        l.linfo_h = plan.linfo;
+        l.h = plan_slices(plan, rp, lanes, chain);
         long long most = 0;
         l.cut = split_slices(l.h, sms, most);
         entries += (size_t)most;
@@ -848,10 +881,11 @@ void CpalSolver::alloc_flow() {
         l.desc = arena_.take<int4>(std::max(l.h.n, 1));
         l.rl = arena_.take<int2>(32 * (size_t)std::max(l.h.n, 1));
         l.cta = arena_.take<int>((size_t)flow_grid_ + 1);
+        l.linfo = arena_.take<int4>(std::max(l.nlong, 1));
         l.ci = arena_.take<int>(len);
         if (flow_smem_[0]) l.v32 = arena_.take<float>(len);
         if (flow_smem_[1]) l.v64 = arena_.take<double>(len);
-        l.part = arena_.take<ulonglong2>(8 * (size_t)std::max((q ? A_ : At_).it.hp.npieces, 1));
+        l.part = arena_.take<ulonglong2>(8 * (size_t)std::max(l.npieces, 1));
     }
     flow_xt_ = arena_.take<ulonglong2>((size_t)n_ << flow_shift_[0]);
     flow_ut_ = arena_.take<ulonglong2>((size_t)m_ << flow_shift_[1]);
@@ -872,7 +906,8 @@ void CpalSolver::upload_flow() {
         up(l.desc, l.h.desc);
         up(l.rl, l.h.rl);
         up(l.cta, l.cut);
-        k_slice_pack<<<grid_for(32LL * l.h.n), kThreads, 0, stream_>>>(l.h.n, l.desc, l.rl, M.it.d.linfo, S_it_, M.rp,
+        up(l.linfo, l.linfo_h);
+        k_slice_pack<<<grid_for(32LL * l.h.n), kThreads, 0, stream_>>>(l.h.n, l.desc, l.rl, l.linfo, l.S, M.rp,
                                                                       (const int *)M.ci, l.ci);
         PDAL_LAUNCH_CHECK();
     }
@@ -887,8 +922,7 @@ void CpalSolver::pack_flow() {
         const int g = grid_for(32LL * l.h.n);
         auto pack = [&](auto *to) {
             if (!to) return;
-            k_slice_pack<<<g, kThreads, 0, stream_>>>(l.h.n, l.desc, l.rl, M.it.d.linfo, S_it_, M.rp,
-                                                      (const double *)M.v, to);
+            k_slice_pack<<<g, kThreads, 0, stream_>>>(l.h.n, l.desc, l.rl, l.linfo, l.S, M.rp, (const double *)M.v, to);
             PDAL_LAUNCH_CHECK();
             launches += 1;
         };
@@ -904,8 +938,7 @@ void CpalSolver::clear_flow() {
     PDAL_CUDA(cudaMemsetAsync(flow_ut_, 0, sizeof(ulonglong2) * ((size_t)m_ << flow_shift_[1]), stream_));
     PDAL_CUDA(cudaMemsetAsync(flow_sums_, 0, sizeof(ulonglong2) * 32 * (size_t)flow_grid_, stream_));
     for (int q = 0; q < 2; ++q)
-        PDAL_CUDA(cudaMemsetAsync(sl_[q].part, 0,
-                                  sizeof(ulonglong2) * 8 * (size_t)std::max((q ? A_ : At_).it.hp.npieces, 1), stream_));
+        PDAL_CUDA(cudaMemsetAsync(sl_[q].part, 0, sizeof(ulonglong2) * 8 * (size_t)std::max(sl_[q].npieces, 1), stream_));
 }
 
 template <typename T>
@@ -913,8 +946,8 @@ SliceDev<T> CpalSolver::slice_dev(int q) const {
     const Sliced &l = sl_[q];
     const DevMatrix &M = q ? A_ : At_;
     const void *val = sizeof(T) == 8 ? (const void *)l.v64 : (const void *)l.v32;
-    return SliceDev<T>{l.desc, l.rl, l.ci, (const T *)val, l.cta, M.it.d.linfo, M.rp,
-                       (typename Tagged<T>::Word *)l.part, l.h.n, M.it.d.nlong, S_it_, O_.persistent_loop == 1};
+    return SliceDev<T>{l.desc, l.rl, l.ci, (const T *)val, l.cta, l.linfo, M.rp,
+                       (typename Tagged<T>::Word *)l.part, l.h.n, l.nlong, l.S, O_.persistent_loop == 1};
 }
 
 /* a cooperative launch of one CTA per SM (also inside a stream capture) */

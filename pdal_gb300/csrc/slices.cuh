@@ -36,21 +36,35 @@
  *          rounds repeat every gather, which costs more than it saves once
  *          the gathers themselves, 32-byte sectors of L2, take the time.
  *
- * Microseconds per iteration (random LPs, 8 nonzeros per column, GB300):
- *   nonzeros  form    launches  tagged  barrier
- *    4,800    FP64      7.7       4.7     6.7
- *             FP32      5.2       3.1     4.6
- *   40,000    FP64     10.6       6.9     8.6
- *             FP32      5.8       4.2     5.8
- *  120,000    FP64     16.9      13.5    12.8
- *             FP32      7.0       9.3     8.1
- *  400,000    FP64     17.5      19.0    15.8
- *             FP32      9.1      17.3     9.8
- *  1,000,000  FP64     38.2      27.0    22.0
- *             FP32     17.4      25.5    14.6
+ * Microseconds per iteration (random LPs, k nonzeros per column, 0.4 rows per
+ * column, GB300):
+ *   nonzeros  k  form    launches  tagged  barrier
+ *     20,000  8  FP64       7.8      5.1     6.8
+ *                FP32       5.5      2.9     4.7
+ *     60,000  1  FP64      10.4      7.5     8.6
+ *                FP32       5.9      5.6     5.0
+ *     60,000  8  FP64      10.9      5.3     7.5
+ *                FP32       6.1      3.0     5.1
+ *    100,000  8  FP64      14.1      7.6     9.0
+ *                FP32       6.6      3.3     5.8
+ *    200,000  1  FP64      17.2     18.4    20.1
+ *                FP32       7.7     10.0     8.1
+ *    200,000  8  FP64      15.0     10.4    10.8
+ *                FP32       7.0      9.3     7.0
+ *    400,000  8  FP64      16.9     12.4    12.6
+ *                FP32       8.7     12.5     8.9
+ *    700,000  8  FP64      29.4     25.1    18.8
+ *                FP32      14.2     22.4    13.4
+ *  1,000,000  2  FP64      55.3     39.6    40.0
+ *                FP32      18.0     21.3    17.0
+ *  1,000,000  8  FP64      38.8     27.8    20.8
+ *                FP32      17.8     23.5    14.6
+ *  1,000,000 20  FP64      34.2     21.0    20.2
+ *                FP32      15.5     20.8    17.6
  * (CpalSolver::flow_form holds the lines drawn from these.)  The tagged power
- * iteration, k_power_flow, takes 6.3 / 7.0 / 11.5 / 15.6 / 23.9 us a step in
- * FP64 where five launches took 17.6 / 18.8 / 21.6 / 24.0 / 36.4.
+ * iteration, k_power_flow, takes 6.7 / 7.0 / 8.0 / 10.5 / 24.2 us a step at
+ * 20,000 / 100,000 / 200,000 / 400,000 / 1,000,000 nonzeros of k = 8, where five
+ * launches take 17.0 / 20.9 / 22.6 / 25.2 / 37.8.
  */
 #pragma once
 
