@@ -381,6 +381,9 @@ class CpalSolver {
     }
 
   public:
+    /* this solver's work only: a synchronisation of the device fails while
+     * another thread's solver captures, and breaks its capture */
+    void wait() const { PDAL_CUDA(cudaStreamSynchronize(stream_)); }
     int panel_rows() const { return use_panels_ ? pan_host_.H : 0; }
     int panels() const { return use_panels_ ? pan_host_.P : 0; }
 
@@ -2774,7 +2777,7 @@ cp_al_gb300_session_t *cp_al_gb300_session_create(const lp_problem_t *prob, cons
         sess->solver.reset(new pdal::CpalSolver(&sess->prob_copy, &local, &o));
         sess->solver->prepare();
         sess->solver->upload();
-        PDAL_CUDA(cudaDeviceSynchronize());
+        sess->solver->wait();
         return sess;
     } catch (const std::exception &e) {
         set_error(e.what());
@@ -2789,7 +2792,7 @@ int cp_al_gb300_session_solve(cp_al_gb300_session_t *s, cp_al_result_t *summary)
         s->solver->setup_device();
         s->solver->run_loop();
         s->solver->result_on_device();
-        PDAL_CUDA(cudaDeviceSynchronize());
+        s->solver->wait();
         if (summary) s->solver->download(summary, false);
         fill_stats(*s->solver, pdal::now_sec() - t0);
         return 0;
@@ -2834,7 +2837,7 @@ int cp_al_gb300_session_iterate(cp_al_gb300_session_t *s, int iterations, cp_al_
         }
         const double t0 = pdal::now_sec();
         if (s->solver->extend(iterations)) s->solver->run_loop();
-        PDAL_CUDA(cudaDeviceSynchronize());
+        s->solver->wait();
         if (summary) s->solver->download(summary, false);
         fill_stats(*s->solver, pdal::now_sec() - t0);
         return 0;

@@ -1,0 +1,67 @@
+"""Solves from several host threads at a time, each with its own session or problem."""
+import threading
+
+import numpy as np
+import pytest
+
+from pdal_gb300 import instances as I, lp
+
+
+def _run(jobs):
+    """Every job in a thread of its own; the first exception is raised here."""
+    out, errors = [None] * len(jobs), []
+
+    def work(i):
+        try:
+            out[i] = jobs[i]()
+        except Exception as e:  # noqa: BLE001 - reported by the caller's thread
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    if errors:
+        raise errors[0]
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("loop", [-1, 0], ids=["resident", "launches"])
+@pytest.mark.parametrize("precision", ["fp64", "fp32_refine"])
+def test_sessions_in_threads(lp_lib, precision, loop):
+    """Eight sessions solved again and again at the same time: the iterates of
+    each are those of its solve alone."""
+    p = {"eps": 1e-14, "iteration_limit": 400, "sv_max_iter": 100}
+    o = {"precision": precision, "fp32_switch_tol": 1e-14, "fp32_stall_evals": 0, "persistent_loop": loop}
+    sessions = [lp.LPSession(I.random_lp(300 + 100 * i, 800 + 250 * i, 8, seed=i), p, o) for i in range(8)]
+    alone = []
+    for s in sessions:
+        s.solve()
+        alone.append(s.fetch())
+
+    def job(s):
+        def solves():
+            for _ in range(6):
+                s.solve()
+            return s.fetch()
+        return solves
+
+    together = _run([job(s) for s in sessions])
+    for s in sessions:
+        s.close()
+    for a, b in zip(alone, together):
+        assert all(np.array_equal(u, v) for u, v in zip(a, b))
+
+
+@pytest.mark.gpu
+def test_solves_from_host_arrays_in_threads(lp_lib):
+    """The same through lp.solve, which allocates and frees on the way, with one
+    LP in the barrier form among small ones."""
+    p = {"eps": 1e-14, "iteration_limit": 400, "sv_max_iter": 100}
+    data = [I.random_lp(300 + 100 * i, 800 + 250 * i, 8, seed=i) for i in range(5)] + [I.random_lp(12000, 30000, 8, seed=9)]
+    alone = [lp.solve(d, p, {}) for d in data]
+    together = _run([lambda d=d: [lp.solve(d, p, {}) for _ in range(3)][-1] for d in data])
+    for a, b in zip(alone, together):
+        assert np.array_equal(a.x, b.x) and np.array_equal(a.y, b.y)
