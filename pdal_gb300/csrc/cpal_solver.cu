@@ -313,6 +313,7 @@ class CpalSolver {
         ulonglong2 *part = nullptr; /* of the precision that iterates */
     } sl_[2];
     int flow_grid_ = 0;             /* CTAs of the resident launches */
+    int flow_warps_ = 0;            /* their warps */
     int flow_shift_[2] = {0, 0};    /* spacing of the tagged x-bar and u */
     template <typename T>
     TaggedVec<T> tagged_x() const {
@@ -824,7 +825,7 @@ void CpalSolver::setup_staged() {
 }
 
 void CpalSolver::plan_flow() {
-    flow_grid_ = 0;
+    flow_grid_ = flow_warps_ = 0;
     flow_smem_[0] = flow_smem_[1] = 0;
     if (O_.persistent_loop == 0 || m_ == 0 || nnz_ == 0 || use_panels_ || O_.primal_staged >= 0) return;
     int dev = 0, sms = 0, coop = 0;
@@ -869,7 +870,15 @@ void CpalSolver::plan_flow() {
         long long most = 0;
         l.cut = split_slices(l.h, sms, most);
         entries += (size_t)most;
+        for (int b = 0; b < sms; ++b) flow_warps_ = std::max(flow_warps_, l.cut[b + 1] - l.cut[b]);
     }
+    /* a warp per slice and no more, since a CTA of 16 takes an SM's registers:
+     * so the solves of several threads run side by side where they are small (ms
+     * a solve of 1 / 2 / 4 / 8 threads, 2,000 x 5,000 in FP64: with 16 warps 5.0 /
+     * 4.6 / 4.4 / 4.3, so 5.0 / 2.7 / 2.0 / 2.0, by launches 10.7 / 6.2 / 3.8 /
+     * 3.1; 20,000 x 50,000, which needs the 16: 10.2 / 9.8 / 9.7 / 9.8, by
+     * launches 16.1 / 11.0 / 7.4 / 6.9) */
+    flow_warps_ = std::min(std::max(flow_warps_, 4), kFlowWarps);
     for (int f = first; f < 2; ++f)
         if (bytes(f, entries) <= kFlowSmem) flow_smem_[f] = std::max<size_t>(bytes(f, entries), 16);
     if (!flow_smem_[0] && !flow_smem_[1])
@@ -1322,7 +1331,7 @@ void CpalSolver::power_iteration() {
     launches += 1;
     if (flow) {
         clear_flow();
-        launch_coop(has_long() ? k_power_flow<true> : k_power_flow<false>, (kFlowWarps + 1) * 32, flow_smem_[1], power_args(),
+        launch_coop(has_long() ? k_power_flow<true> : k_power_flow<false>, (flow_warps_ + 1) * 32, flow_smem_[1], power_args(),
                     std::min(h.max_iter, INT32_MAX - 8));
         launches += 1;
         PDAL_CUDA(cudaMemcpyAsync(h_ps_, ps_, sizeof(PowerState), cudaMemcpyDeviceToHost, stream_));
@@ -1804,11 +1813,11 @@ void CpalSolver::launch_flow(int F) {
         PDAL_CUDA(cudaMemsetAsync(flow_bar_, 0, sizeof(unsigned), stream_));
         launch_coop(has_long() ? (beta_on_ ? k_flow<T, true, true, true> : k_flow<T, false, true, true>)
                                : (beta_on_ ? k_flow<T, true, true, false> : k_flow<T, false, true, false>),
-                    kFlowWarps * 32, smem, L);
+                    flow_warps_ * 32, smem, L);
     } else {
         launch_coop(has_long() ? (beta_on_ ? k_flow<T, true, false, true> : k_flow<T, false, false, true>)
                                : (beta_on_ ? k_flow<T, true, false, false> : k_flow<T, false, false, false>),
-                    kFlowWarps * 32, smem, L);
+                    flow_warps_ * 32, smem, L);
     }
 }
 

@@ -72,7 +72,7 @@
 
 namespace pdal {
 
-constexpr int kFlowWarps = 16; /* warps of a CTA that work on slices */
+constexpr int kFlowWarps = 16; /* warps of a CTA that work on slices, at most (the launch says how many) */
 
 /* ------------------------------------------------------------------ */
 /* tagged words                                                        */
@@ -141,9 +141,9 @@ struct FlowGuard {
     }
 };
 
-/* Grid barrier of the worker warps (for the problems whose gathers are too
+/* Grid barrier (for the problems whose gathers are too
  * many to poll): one release-add per CTA on a counter that is zero at launch,
- * then an acquire poll until all CTAs of this barrier have arrived.  All worker
+ * then an acquire poll until all CTAs of this barrier have arrived.  All
  * warps of a CTA call every wait(), a warp whose own work gave up (!good) with
  * them: a warp that left by itself would leave its CTA's others in bar.sync for
  * good.  The same wait() then returns false in all of them, without polling. */
@@ -153,11 +153,10 @@ struct FlowBarrier {
     int *failed; /* shared, zero at first */
     FlowGuard guard;
     unsigned target;
-    __device__ __forceinline__ void workers() const { asm volatile("bar.sync 1, %0;" ::"n"(kFlowWarps * 32) : "memory"); }
     __device__ __forceinline__ bool wait(bool good_so_far) {
         target += gridDim.x;
         if (!good_so_far) *(volatile int *)failed = 1;
-        workers();
+        __syncthreads();
         if (threadIdx.x == 0) {
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
             int spins = 0, good = *(volatile int *)failed == 0;
@@ -172,7 +171,7 @@ struct FlowBarrier {
             }
             *ok = good;
         }
-        workers();
+        __syncthreads();
         return *ok != 0;
     }
 };
@@ -410,7 +409,7 @@ __device__ __noinline__ bool flow_long_sum(const typename Tagged<T>::Word *part,
  * Returns false for the whole warp when a wait gave up. */
 template <bool LONG, typename T, class Src, class Epi, class Wait>
 __device__ __forceinline__ bool flow_phase(const SliceDev<T> &M, const SliceShare<T> &sh, const Src &src, Epi &epi,
-                                           unsigned tag, const FlowGuard &guard, Wait wait) {
+                                           unsigned tag, const FlowGuard &guard, int warps, Wait wait) {
     const int lane = threadIdx.x & 31, first = sh.s0 + (int)(threadIdx.x >> 5);
     int4 d = sh.d;
     int2 e = sh.e;
@@ -418,7 +417,7 @@ __device__ __forceinline__ bool flow_phase(const SliceDev<T> &M, const SliceShar
     typename Epi::In in;
     if (lead) in = epi.fetch(e.x);
     if (!wait()) return false;
-    for (int s = first; s < sh.s1; s += kFlowWarps) {
+    for (int s = first; s < sh.s1; s += warps) {
         if (s != first) {
             d = M.desc[s];
             e = M.rl[(size_t)s * 32 + lane];
@@ -440,7 +439,7 @@ __device__ __forceinline__ bool flow_phase(const SliceDev<T> &M, const SliceShar
     }
     if constexpr (LONG) {
         if (M.nlong == 0) return true;
-        for (int s = first; s < sh.s1; s += kFlowWarps) {
+        for (int s = first; s < sh.s1; s += warps) {
             const int4 d = M.desc[s];
             if (d.z > 0) continue;
             const int4 li = M.linfo[M.rl[(size_t)s * 32].x]; /* {row, pieces, first piece, first entry} */
@@ -567,6 +566,7 @@ __global__ void __launch_bounds__(kFlowWarps * 32, 1) k_flow(FlowArgs<T> L) {
     __syncthreads();
     FlowBarrier bar{L.bar, &bar_ok, &bar_failed, L.guard, 0u};
     auto none = [] { return true; };
+    const int warps = (int)(blockDim.x >> 5);
     bool good = true; /* no wait of this warp has given up */
     for (int i = 1; i <= L.F; ++i) {
         const T w = L.wt[i].w, omw = L.wt[i].omw;
@@ -583,15 +583,15 @@ __global__ void __launch_bounds__(kFlowWarps * 32, 1) k_flow(FlowArgs<T> L) {
                 return !left;
             };
             auto wait_next = [&] { return i == 1 || wait(); };
-            good = flow_phase<LONG, T>(L.at, sp, PlainSource<T>{L.gat}, ep, tag, L.guard, wait_next);
-            if (!left) good = flow_phase<LONG, T>(L.a, sd, PlainSource<T>{L.pa.xbar}, ed, tag, L.guard, wait);
+            good = flow_phase<LONG, T>(L.at, sp, PlainSource<T>{L.gat}, ep, tag, L.guard, warps, wait_next);
+            if (!left) good = flow_phase<LONG, T>(L.a, sd, PlainSource<T>{L.pa.xbar}, ed, tag, L.guard, warps, wait);
             if (left) break;
         } else {
             if (i == 1)
-                good = flow_phase<LONG, T>(L.at, sp, PlainSource<T>{L.gat}, ep, tag, L.guard, none);
+                good = flow_phase<LONG, T>(L.at, sp, PlainSource<T>{L.gat}, ep, tag, L.guard, warps, none);
             else
-                good = flow_phase<LONG, T>(L.at, sp, TaggedSource<T>{L.ut, tag - 1, L.guard}, ep, tag, L.guard, none);
-            good = good && flow_phase<LONG, T>(L.a, sd, TaggedSource<T>{L.xt, tag, L.guard}, ed, tag, L.guard, none);
+                good = flow_phase<LONG, T>(L.at, sp, TaggedSource<T>{L.ut, tag - 1, L.guard}, ep, tag, L.guard, warps, none);
+            good = good && flow_phase<LONG, T>(L.a, sd, TaggedSource<T>{L.xt, tag, L.guard}, ed, tag, L.guard, warps, none);
             if (!good) break;
         }
     }
@@ -654,10 +654,10 @@ __device__ __forceinline__ void flow_publish(FlowSums &f, int active, unsigned r
 
 /* a warp with no rows of A to publish for and no entries in its columns */
 template <typename T>
-__device__ __forceinline__ bool flow_idle(const SliceDev<T> &at, const SliceShare<T> &sp, int active) {
+__device__ __forceinline__ bool flow_idle(const SliceDev<T> &at, const SliceShare<T> &sp, int active, int warps) {
     const int warp = threadIdx.x >> 5;
     if (warp < active) return false;
-    for (int s = sp.s0 + warp; s < sp.s1; s += kFlowWarps)
+    for (int s = sp.s0 + warp; s < sp.s1; s += warps)
         if (at.desc[s].y > 0) return false;
     return true;
 }
@@ -829,10 +829,11 @@ __global__ void __launch_bounds__(kFlowWarps * 32 + 32, 1) k_power_flow(FlowPowe
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const double c1 = L.ps->inv, n1 = L.ps->vsq, tol = L.ps->tol;
-    const int active = max(1, min(sd.s1 - sd.s0, kFlowWarps)); /* warps that publish sums */
+    const int warps = (int)(blockDim.x >> 5) - 1;
+    const int active = max(1, min(sd.s1 - sd.s0, warps)); /* warps that publish sums */
     /* every step whose residual may be wanted, plus the four that follow it */
     const int last = max_steps + 4;
-    if (warp == kFlowWarps) {
+    if (warp == warps) {
         double ck[4], nk[4], s2k[4]; /* by step & 3 */
         ck[1] = c1;
         nk[1] = n1;
@@ -865,7 +866,7 @@ __global__ void __launch_bounds__(kFlowWarps * 32 + 32, 1) k_power_flow(FlowPowe
         }
         return;
     }
-    if (flow_idle(L.at, sp, active)) return;
+    if (flow_idle(L.at, sp, active, warps)) return;
     auto none = [] { return true; };
     for (int k = 1; k <= last; ++k) {
         double c = c1, a = 0.0, b = 0.0;
@@ -881,14 +882,14 @@ __global__ void __launch_bounds__(kFlowWarps * 32 + 32, 1) k_power_flow(FlowPowe
         FlowStoreEpi ec{L.dt, (unsigned)k, c};
         bool ok;
         if (k == 1)
-            ok = flow_phase<LONG, double>(L.at, sp, PlainSource<double>{L.v0}, ec, (unsigned)k, L.guard, none);
+            ok = flow_phase<LONG, double>(L.at, sp, PlainSource<double>{L.v0}, ec, (unsigned)k, L.guard, warps, none);
         else
             ok = flow_phase<LONG, double>(L.at, sp, TaggedSource<double>{L.vt, (unsigned)(k - 1), L.guard}, ec, (unsigned)k,
-                               L.guard, none);
+                               L.guard, warps, none);
         double s[4] = {0.0, 0.0, 0.0, 0.0};
         FlowPowerEpi er{L, (unsigned)k, a, b, s};
         ok = ok && flow_phase<LONG, double>(L.a, sd, TaggedSource<double>{L.dt, (unsigned)k, L.guard}, er, (unsigned)k,
-                                 L.guard, none);
+                                 L.guard, warps, none);
         if (!ok) return;
         if (warp < active) flow_publish(f, active, (unsigned)k, s, L.sums + (size_t)(k & 3) * gridDim.x * 4);
     }
