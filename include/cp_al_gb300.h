@@ -121,11 +121,14 @@ typedef struct {
     int persistent_loop;          /* LPs whose matrices fit in the shared memory of the GPU's SMs: run an
                                      evaluation block's iterations, and the FP64 power iteration, in one
                                      resident launch each instead of one launch per product.  -1 (default)
-                                     = where that was measured faster (by size and precision; not with
-                                     column panels, an explicit primal_staged or timing); 1 = the
+                                     = where that was measured faster (by size, shape and precision; not
+                                     with column panels, an explicit primal_staged or timing); 1 = the
                                      iterations of every LP that fits, with the launches' summation
                                      order (bit-identical to 0), the power iteration by launches; 0 =
-                                     never */
+                                     never.  A resident launch starts when every SM has room for a block
+                                     of it: up to some 100,000 nonzeros it takes a part of an SM, above
+                                     all of it, and then waits while another stream's kernel holds an SM
+                                     and takes turns with other threads' solves (0 does not) */
     int dual_fused_finish;        /* with the panel path: the group that writes a long row's last panel
                                      partial also sums the row's partials (fixed order) and runs its
                                      dual epilogue, instead of a separate launch.  1 = fused; 0 or -1

@@ -151,6 +151,8 @@ struct IterVecs {
 /* Resident launches need the packed matrices of both products in the shared
  * memory of one CTA per SM, in the precision that iterates. */
 constexpr size_t kFlowSmem = 224 * 1024;
+static_assert(kFlowSmem + sizeof(FlowSums) + 4 * sizeof(FlowScalars) + 64 <= 227 * 1024,
+              "a CTA fits on every SM, so that a launch of one per SM is never refused");
 /* Rows of up to this many entries sit in the lanes of one warp, also where the
  * row blocks of a small LP are shorter: a longer one costs its eight warps an
  * exchange per piece. */
