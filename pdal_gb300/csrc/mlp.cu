@@ -766,9 +766,25 @@ struct Mlp {
         fill(oW1, (size_t)in * h, in);
         fill(oW2, (size_t)h * h, h);
         fill(oW3, (size_t)h * out, h);
-        PDAL_CUDA(cudaMemcpy(P.p, init.data(), np * 4, cudaMemcpyHostToDevice));
-        PDAL_CUDA(cudaMemset(Ma.p, 0, np * 4));
-        PDAL_CUDA(cudaMemset(Va.p, 0, np * 4));
+        set_params(init.data());
+    }
+    /* Copies run on the handle's stream, which no other stream orders: what the
+     * legacy stream holds of other work neither delays them past the products
+     * that read them nor waits for these. */
+    void put(float *dst, const float *src, size_t count) {
+        PDAL_CUDA(cudaMemcpyAsync(dst, src, count * 4, cudaMemcpyHostToDevice, s));
+    }
+    void get(float *dst, const float *src, size_t count) {
+        PDAL_CUDA(cudaMemcpyAsync(dst, src, count * 4, cudaMemcpyDeviceToHost, s));
+        PDAL_CUDA(cudaStreamSynchronize(s));
+    }
+    /* new parameters, the moments of their updates zero */
+    void set_params(const float *params) {
+        put(P.p, params, np);
+        PDAL_CUDA(cudaStreamSynchronize(s));
+        PDAL_CUDA(cudaMemsetAsync(Ma.p, 0, np * 4, s));
+        PDAL_CUDA(cudaMemsetAsync(Va.p, 0, np * 4, s));
+        adam_t = 0;
     }
     ~Mlp() {
         if (s) cudaStreamDestroy(s);
@@ -925,7 +941,7 @@ long long pdal_mlp_num_params(const pdal_mlp_t *h) { return h ? (long long)h->m-
 int pdal_mlp_get_params(const pdal_mlp_t *h, float *params) {
     if (!h || !params) return fail("pdal_mlp_get_params: NULL argument");
     try {
-        PDAL_CUDA(cudaMemcpy(params, h->m->P.p, h->m->np * 4, cudaMemcpyDeviceToHost));
+        h->m->get(params, h->m->P.p, h->m->np);
         return 0;
     } catch (const std::exception &e) {
         return fail(e.what());
@@ -935,10 +951,7 @@ int pdal_mlp_get_params(const pdal_mlp_t *h, float *params) {
 int pdal_mlp_set_params(pdal_mlp_t *h, const float *params) {
     if (!h || !params) return fail("pdal_mlp_set_params: NULL argument");
     try {
-        PDAL_CUDA(cudaMemcpy(h->m->P.p, params, h->m->np * 4, cudaMemcpyHostToDevice));
-        PDAL_CUDA(cudaMemset(h->m->Ma.p, 0, h->m->np * 4));
-        PDAL_CUDA(cudaMemset(h->m->Va.p, 0, h->m->np * 4));
-        h->m->adam_t = 0;
+        h->m->set_params(params);
         return 0;
     } catch (const std::exception &e) {
         return fail(e.what());
@@ -951,8 +964,9 @@ int pdal_mlp_set_data(pdal_mlp_t *h, int n, const float *X, const float *Y) {
         pdal::Mlp &m = *h->m;
         m.Xd.ensure((size_t)n * m.in);
         m.Yd.ensure((size_t)n * m.out);
-        PDAL_CUDA(cudaMemcpy(m.Xd.p, X, (size_t)n * m.in * 4, cudaMemcpyHostToDevice));
-        PDAL_CUDA(cudaMemcpy(m.Yd.p, Y, (size_t)n * m.out * 4, cudaMemcpyHostToDevice));
+        m.put(m.Xd.p, X, (size_t)n * m.in);
+        m.put(m.Yd.p, Y, (size_t)n * m.out);
+        PDAL_CUDA(cudaStreamSynchronize(m.s));
         m.ndata = n;
         return 0;
     } catch (const std::exception &e) {
@@ -1007,7 +1021,7 @@ double pdal_mlp_loss_grad(pdal_mlp_t *h, int n, const float *X, const float *Y, 
         A.grad = m.G.p;
         m.step(n, m.Xb.p, m.Yb.p, nullptr, A, grad != nullptr);
         const double loss = m.read_loss();
-        if (grad) PDAL_CUDA(cudaMemcpy(grad, m.G.p, m.np * 4, cudaMemcpyDeviceToHost));
+        if (grad) m.get(grad, m.G.p, m.np);
         return loss;
     } catch (const std::exception &e) {
         return fail(e.what());
