@@ -187,7 +187,8 @@ typedef struct {
     int dual_concurrent;          /* with the panel path: the dual step's short-row launch and its
                                      long rows' panel launch run concurrently on two streams (also in
                                      the captured graphs).  1 and -1 (default) = yes (an iteration of
-                                     the large LP: FP32 98.9 -> 97 us, FP64 183 -> 178 us), 0 = one
+                                     the 1M x 2M power-law LP: FP32 187.8 -> 185.0 us, FP64 376.9 ->
+                                     373.8; of half its size 98.4 -> 92.4, 200.4 -> 192.1), 0 = one
                                      after the other.  Results are bit-identical either way */
     int resident_fail_launch;     /* fault injection for tests: this resident launch of the solver (1 = the
                                      first, in the order they are issued or captured) gives up at the

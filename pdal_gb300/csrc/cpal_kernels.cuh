@@ -622,6 +622,7 @@ struct PanelDev {
      * per long row (zero between launches) and segments per long row */
     unsigned *cnt;
     const int *nseg;
+    bool prefetch; /* the matrix to L2 ahead of its loads */
 };
 
 constexpr int kPanelThreads = 512;
@@ -705,9 +706,13 @@ __global__ void __launch_bounds__(kPanelThreads, sizeof(T) == 4 ? 2 : 1) k_dual_
     T *sx = reinterpret_cast<T *>(panel_smem);
     const int4 c = pd.cta[blockIdx.x];
     /* the block's share of the matrix comes to L2 while x-bar is waited for
-     * and staged (large LP, FP32 iteration 98.8 -> 96.9 us): the segments of
-     * consecutive pieces are consecutive */
-    if (threadIdx.x == 0 && c.x < c.y) {
+     * and staged, where the whole matrix takes a third of L2 at most: the
+     * segments of consecutive pieces are consecutive.  An iteration of the
+     * power-law LP, FP32 / FP64: 250,000 x 500,000 (24 / 40 MB) 63.7 -> 60.0 /
+     * 119.7 -> 112.9 us, 500,000 x 1M (48 / 80 MB) 92.4 -> 94.1 / 192.1 ->
+     * 194.5, 1M x 2M 185.0 -> 189.4 / 373.8 -> 377.1: a larger one only drives
+     * out what the short rows' blocks gather. */
+    if (pd.prefetch && threadIdx.x == 0 && c.x < c.y) {
         const int k0 = pd.seg[pd.piece[c.x].y].y, k1 = pd.seg[pd.piece[c.y - 1].z - 1].z;
         prefetch_l2(pd.val + k0, sizeof(T) * (size_t)(k1 - k0));
         prefetch_l2(pd.off + k0, sizeof(uint16_t) * (size_t)(k1 - k0));
