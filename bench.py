@@ -283,8 +283,8 @@ def run_ours(args, rank, world, local):
     sp = {"eps": 1e-6, "l_inf_ruiz_iterations": 4}
     kkt = {}
     for tag, opts in (("chosen", {"precision": "fp32_refine", "device": local}), ("plain_fp64", {"device": local}),
-                      ("chosen_device_loop", {"precision": "fp32_refine", "device": local, "persistent_loop": 1}),
-                      ("plain_fp64_device_loop", {"device": local, "persistent_loop": 1})):
+                      ("chosen_resident_launch_order", {"precision": "fp32_refine", "device": local, "persistent_loop": 1}),
+                      ("plain_fp64_resident_launch_order", {"device": local, "persistent_loop": 1})):
         lp.solve(small, sp, opts)
         runs = []
         for _ in range(3):

@@ -834,6 +834,7 @@ void CpalSolver::plan_flow() {
     flow_grid_ = flow_warps_ = 0;
     flow_smem_[0] = flow_smem_[1] = 0;
     if (O_.persistent_loop == 0 || m_ == 0 || nnz_ == 0 || use_panels_ || O_.primal_staged >= 0) return;
+    if ((long long)m_ + n_ > 4LL * nnz_ + 4096) return; /* mostly empty rows, which a plan lists one by one */
     int dev = 0, sms = 0, coop = 0;
     PDAL_CUDA(cudaGetDevice(&dev));
     PDAL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -1292,8 +1293,8 @@ FlowPowerArgs CpalSolver::power_args() {
 
 /* The start vector of the sigma_max estimates, std::normal_distribution over
  * std::mt19937(1) as the reference draws it in a fresh process
- * (LP/CP_AL/src/utils.cu:27-28, 102-106), on the device (k_mt_*); the launches
- * draw 1.4 words per word needed on average and a margin of ten deviations. */
+ * (LP/CP_AL/src/utils.cu:27-28, 102-106), on the device (k_mt_*), from the
+ * words needed on average and a margin of ten deviations (mt_twists). */
 void CpalSolver::start_vector(double *v) {
     const int blocks = mt_blocks(m_), pairs = 156 * mt_twists(m_);
     MtSeed seed;

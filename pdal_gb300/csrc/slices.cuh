@@ -9,13 +9,13 @@
  * warp's loads of column indices and values are whole 128-byte lines and no
  * staging, row pointers or block barriers stand between a load and its
  * product.  Rows are sorted by length within a window, so the lanes of a
- * slice end together; each has the fewest lanes that give every SM a slice, and
- * more where it is long, since a lane's entries are dependent rounds of gathers.
- * Few lanes matter most in FP64: an FP64 instruction holds an SM's FP64 pipe
- * for 19 cycles however many lanes are active, and a dependent one waits 64
- * (measured), so with the row-block engine's 16 lanes a row the epilogues, in
- * two lanes of a warp, bounded the iteration of a small LP.  (persistent_loop
- * = 1 keeps that engine's lanes and summation order: bit-identical sums.)
+ * slice end together.  Lanes cost and save: a lane's entries are dependent
+ * rounds of gathers, but an FP64 instruction holds an SM's FP64 pipe for 19
+ * cycles however many lanes are active, and a dependent one waits 64 (measured),
+ * so the epilogues of many lanes a row, in a few lanes of a warp, bound the
+ * iteration of an LP that fills the SMs with one (CpalSolver::plan_flow draws
+ * the line).  persistent_loop = 1 keeps the row-block engine's lanes and
+ * summation order: bit-identical sums.
  *
  * k_flow runs the iterations of one evaluation block, with the matrices in
  * the shared memory of one CTA per SM, in one of two forms:
@@ -25,7 +25,7 @@
  *          and a warp that gathers an entry polls it until it carries the
  *          number it needs.  An exchange is one store and the polls that see
  *          it, about 1,800 cycles over the whole GPU, where a grid barrier
- *          and the gather behind it take 2,600 and a launch more.  One buffer
+ *          takes 2,300, without the gather behind it, and a launch more.  One buffer
  *          per vector is enough: an entry x-bar_j is gathered exactly by the
  *          rows with a nonzero in column j, and the next x-bar_j is made from
  *          the u of those rows, each stored after its row has gathered

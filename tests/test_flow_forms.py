@@ -62,3 +62,18 @@ def test_values_are_those_of_the_launches(lp_lib, data):
         assert a.iterations == b.iterations
         for u, v in ((a.x, b.x), (a.y, b.y)):
             assert np.linalg.norm(u - v) <= tol * (1 + np.linalg.norm(u))
+
+
+@pytest.mark.gpu
+def test_mostly_empty_columns_run_by_launches(lp_lib):
+    """6,000 nonzeros in 60,000 columns: a plan of the resident launches would
+    list the empty ones too."""
+    d = I.random_lp(100, 60000, 1, seed=2)
+    rp, ci, v, shape = d.csr()
+    A = sp.csr_matrix((v, ci, rp), shape=shape).tocsc()
+    A.data[np.repeat(np.arange(shape[1]), np.diff(A.indptr)) >= 6000] = 0.0
+    A = A.tocsr()
+    A.eliminate_zeros()
+    d.A = (A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data, shape)
+    r = lp.solve(d, P, _options("fp64"))
+    assert r.iterations == 200 and r.stats["kernel_launches"] > 300
