@@ -266,8 +266,9 @@ __device__ void blk_equilibrate(const BInst &I, const BOpts &o, CpalState &s, do
 }
 
 /* The scale goes onto the column sums, once per column, and onto the quotient,
- * once: an FP64 instruction per nonzero less in a step that the FP64 pipe and the
- * staging bound (300 LPs of 50 to 5,000 rows: 819 -> 783 ms). */
+ * once: an FP64 instruction per nonzero less (the FP64 pipe is 38% busy in a block;
+ * latency of staging and barriers bounds the rest).  300 LPs of 50 to 5,000 rows: 816
+ * -> 787 ms, 2 or 3 times what two runs of one side differ. */
 struct PowColEpiB : NoLongRed {
     double *dp, inv;
     __device__ __forceinline__ void operator()(int j, const double *s, Red<0, 0> &) const { dp[j] = inv * s[0]; }

@@ -337,28 +337,38 @@ class CpalSolver {
     /* How the iteration's products run.  The lines lie where the measured
      * times cross (the table in slices.cuh; `rows`: rows and columns, whose
      * epilogues bound every form where there are few nonzeros to each).
-     * FP64: polling pays up to 200,000 nonzeros, the barrier form above; LPs of
-     * fewer nonzeros than rows gain up to 150,000 and nothing beyond, those of
-     * more than 250,000 rows nothing before the launches' row blocks grow.
+     * FP64: polling pays up to 200,000 nonzeros, and where there are some two to
+     * a row at every size, the barrier form elsewhere; LPs of fewer nonzeros than
+     * rows gain up to 150,000 and nothing beyond, those of more than 250,000 rows
+     * nothing before the launches' row blocks grow.
      * FP32, whose launches take half the time: polling up to 100,000 nonzeros
      * where there are 1.5 or more to a row, up to 30,000 otherwise, where the
-     * barrier form gains to 150,000; and the barrier form from 630,000 on where
-     * a lane per row fills the warps (fewer rows have chains that the launches
-     * cut shorter).  `timing` brackets single launches. */
+     * barrier form gains to 150,000; and the barrier form from 630,000 to
+     * 1,500,000 where a lane per row fills the warps with up to 32 entries each
+     * (fewer rows, and longer ones, have chains that the launches cut shorter,
+     * and with more nonzeros the SMs have three slices a warp: 1.2M nonzeros of 8
+     * per column 16.0 against 17.7 us, 2M 35.5 against 27.4).  `timing` brackets
+     * single launches. */
     template <typename T>
     Flow flow_form() const {
-        if (flow_smem_[sizeof(T) == 8] == 0 || O_.timing != 0) return Flow::launches;
+        return flow_smem_[sizeof(T) == 8] == 0 ? Flow::launches : flow_rule<T>();
+    }
+    template <typename T>
+    Flow flow_rule() const {
+        if (O_.timing != 0) return Flow::launches;
         if (O_.persistent_loop == 1) return Flow::tagged;
         const long long rows = (long long)m_ + n_;
         if (sizeof(T) == 8) {
             if (nnz_ > 150000 && (rows > nnz_ || (rows > 250000 && nnz_ <= 600000))) return Flow::launches;
-            return nnz_ <= 200000 ? Flow::tagged : Flow::barrier;
+            return nnz_ <= 200000 || 10LL * nnz_ < 21 * rows ? Flow::tagged : Flow::barrier;
         }
         if (nnz_ <= 30000) return Flow::tagged;
         if (2LL * nnz_ < 3 * rows && nnz_ <= 150000) return Flow::barrier;
         if (nnz_ <= 100000) return Flow::tagged;
-        const bool filled = 2LL * std::min(m_, n_) > 32LL * kFlowSlices * flow_grid_;
-        return nnz_ >= 630000 && 5LL * nnz_ >= 7 * rows && filled ? Flow::barrier : Flow::launches;
+        const long long shorter = std::min(m_, n_);
+        const bool filled = 2 * shorter > 32LL * kFlowSlices * flow_grid_ && nnz_ <= 32 * shorter;
+        return nnz_ >= 630000 && nnz_ <= 1500000 && 10LL * nnz_ >= 19 * rows && filled ? Flow::barrier
+                                                                                      : Flow::launches;
     }
     template <typename T>
     SliceDev<T> slice_dev(int which) const;
@@ -846,8 +856,12 @@ void CpalSolver::plan_flow() {
      * exchange alone: 26,900 cycles packed, 6,600 with 128 bytes per entry) */
     for (int q = 0; q < 2; ++q) flow_shift_[q] = (q ? m_ : n_) <= 1024 ? 4 : (q ? m_ : n_) <= 4096 ? 2 : 0;
     auto bytes = [](int f, size_t entries) { return entries * (sizeof(int) + (f ? 8 : 4)); };
-    const int first = fp32_phase_ ? 0 : 1;
-    if (bytes(first, 2 * (size_t)nnz_) > sms * kFlowSmem) return;
+    /* the precisions that would use the plan: FP32 for its iterations, FP64 also
+     * for its power iteration, which gains wherever it fits */
+    bool want[2] = {fp32_phase_ && flow_rule<float>() != Flow::launches,
+                    (!fp32_phase_ && O_.persistent_loop != 1) || flow_rule<double>() != Flow::launches};
+    for (int f = 0; f < 2; ++f) want[f] = want[f] && bytes(f, 2 * (size_t)nnz_) <= sms * kFlowSmem;
+    if (!want[0] && !want[1]) return;
     size_t entries = 0; /* of a CTA */
     for (int q = 0; q < 2; ++q) {
         Sliced &l = sl_[q];
@@ -886,8 +900,8 @@ void CpalSolver::plan_flow() {
      * 3.1; 20,000 x 50,000, which needs the 16: 10.2 / 9.8 / 9.7 / 9.8, by
      * launches 16.1 / 11.0 / 7.4 / 6.9) */
     flow_warps_ = std::min(std::max(flow_warps_, 4), kFlowWarps);
-    for (int f = first; f < 2; ++f)
-        if (bytes(f, entries) <= kFlowSmem) flow_smem_[f] = std::max<size_t>(bytes(f, entries), 16);
+    for (int f = 0; f < 2; ++f)
+        if (want[f] && bytes(f, entries) <= kFlowSmem) flow_smem_[f] = std::max<size_t>(bytes(f, entries), 16);
     if (!flow_smem_[0] && !flow_smem_[1])
         for (Sliced &l : sl_) l.h = HostSlices();
 }

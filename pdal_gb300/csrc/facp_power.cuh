@@ -2,19 +2,21 @@
  * facp_power.cuh -- the power iterations of the convex QP solver (sigma_max of
  * A, the extreme eigenvalues of Q) in a resident kernel of their own (sm_103a).
  *
- * What bounds a step is the FP64 pipe -- an FP64 instruction holds it for 19
- * cycles however many lanes are active -- and behind it the latency of the
- * gathers.  So a lane owns a row: 32 rows of about equal length make a slice
- * (rows sorted by length within a window of 2,048), stored entry by entry, whose
+ * What bounds a step is latency: two grid barriers, the gathers between them,
+ * and FP64 instructions, which hold the pipe for 19 cycles however many lanes are
+ * active and make a dependent one wait 64 (counters at 50,000 variables: warps at
+ * a barrier 27 of 38 cycles, FP64 pipe 22% busy, L2 22%; at 200,000 FP64 33%, L2
+ * 43%).  So a lane owns a row: 32 rows of about equal length make a slice (rows
+ * sorted by length within a window of 2,048), stored entry by entry, whose
  * products and whose epilogue then run with all lanes active, four gathers in
  * flight per lane, and no shared memory or block barrier in between; what is one
- * number for the grid is computed in one lane.  The
- * persistent iteration kernel (k_facp) sums a row in two to four lanes after
- * staging the products; it keeps the matrices with a row of more than
- * kPowerChain entries, whose lane would be a chain of dependent gathers.
+ * number for the grid is computed in one lane.  The persistent iteration kernel
+ * (k_facp) sums a row in two to four lanes after staging the products; it keeps
+ * the matrices with a row of more than kPowerChain entries, whose lane would be a
+ * chain of dependent gathers.
  * A step for sigma_max of a random 25,000 x 50,000 A with 500,000 nonzeros: 23 ->
- * 14.7 us, 100,000 x 200,000 with 2M: 57 -> 28 us, of which the FP64 pipe needs 10
- * (1,024 threads or two, eight gathers in flight: 10 to 30% slower).
+ * 14.7 us, 100,000 x 200,000 with 2M: 57 -> 28 us (1,024 threads or two, eight
+ * gathers in flight: 10 to 30% slower).
  */
 #pragma once
 

@@ -144,7 +144,8 @@ __global__ void k_finish_scale(int len, double *s, double *cum) {
  * entry, whole lines at a time and every lane with a division of its own, where a
  * thread per row had its 32 lanes in 32 lines and divided for the longest row of
  * the warp; the maxima are integers, since the bits of non-negative doubles order
- * as the numbers do and the FP64 pipe bounds this kernel.  QP of 200,000
+ * as the numbers do, and leave the FP64 pipe to the divisions (42% busy in a pass
+ * that divides; what bounds it is latency).  QP of 200,000
  * variables (3.2M nonzeros and their transposes), equilibration with the host's
  * transposes: 14.4 -> 13.0 ms, of it on the GPU 2.5. */
 __global__ void __launch_bounds__(256) k_equil_rows(int rows, const int *__restrict__ rp, const int *__restrict__ ci,

@@ -31,6 +31,8 @@ def _dense(m, n):
     (10000, 25000, 8, "fp32_refine", False),     # FP32 between 100,000 and 630,000
     (50000, 125000, 8, "fp32_refine", True),
     (20000, 50000, 20, "fp32_refine", False),    # fewer rows than lanes
+    (30000, 70000, 20, "fp32_refine", False),    # long ones
+    (80000, 200000, 8, "fp32_refine", False),    # over 1,500,000
     (280000, 700000, 1, "fp32_refine", False)])
 def test_form_by_size_and_shape(lp_lib, m, n, k, precision, resident):
     """The iterations of a block are one launch, or two each."""
